@@ -142,9 +142,11 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
     int* err = nullptr;
     void* tmp = nullptr;
     size_t tmp_bytes = 0;
+    uint8_t* u8 = nullptr;  // byte copy of integer rows in [0, 255]: a quarter of the gathered bytes
+    int u8_ld = 0;
     auto cleanup = [&]() {
         cudaFree(d_fwd); cudaFree(k0); cudaFree(k1); cudaFree(v0); cudaFree(v1);
-        cudaFree(ctr); cudaFree(err); cudaFree(tmp);
+        cudaFree(ctr); cudaFree(err); cudaFree(tmp); cudaFree(u8);
     };
     if ((e = cudaMalloc(&d_fwd, maxB * sd * sizeof(int32_t))) != cudaSuccess ||
         (e = cudaMalloc(&k0, maxE * 4)) != cudaSuccess || (e = cudaMalloc(&k1, maxE * 4)) != cudaSuccess ||
@@ -160,6 +162,12 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
     e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k0, k1, v0, v1, (int)maxE, 0, key_bits, st);
     if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, 4, st);
+    if (e == cudaSuccess && kind == SONG_KIND_L2 && byte_rows(range, dim)) {
+        u8_ld = u8_row_bytes(dim);
+        e = cudaMalloc(&u8, (size_t)n * u8_ld);
+        if (e == cudaSuccess)
+            e = convert_rows_u8(static_cast<const float*>(d_base), n, dim, ld, u8, u8_ld, st);
+    }
     int64_t s = 1;
     while (e == cudaSuccess && s < n) {
         const int B = (int)std::min<int64_t>(n - s, std::max<int64_t>(1, s / ratio));
@@ -175,7 +183,7 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
         a.dim = dim;
         a.ld = ld;
         a.qld = ld;
-        a.qdim = dim;  // the generic (dim > 256) instance stages this many query floats
+        a.qdim = kind == SONG_KIND_L2 ? ld : dim;
         a.block_size = bs;
         a.k = sd;
         a.nq = B;
@@ -183,10 +191,9 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
         a.bf_words = bf_words;
         a.bf_nhash = 4;
         a.n_multiprobe = 1;  // the reference build search starts from node 0 alone
-        a.int_base = range.int_base;
-        a.base_min = range.lo;
-        a.base_max = range.hi;
-        search_warp_smem(kind, dim, a.cap, bf_words, &a);
+        a.u8 = u8;
+        a.u8_ld = u8_ld;
+        search_warp_smem(kind, a.qdim, a.cap, bf_words, &a);
         e = cudaMemsetAsync(ctr, 0, 4, st);
         if (e == cudaSuccess) e = launch_search(kind, a, num_sms, st);
         if (e != cudaSuccess) break;
@@ -300,7 +307,7 @@ cudaError_t build_graph_with_scratch(int kind, const void* d_base, int64_t n, in
         a.dim = dim;
         a.ld = ld;
         a.qld = ld;
-        a.qdim = dim;  // the generic (dim > 256) instance stages this many query floats
+        a.qdim = kind == SONG_KIND_L2 ? ld : dim;
         a.block_size = bs;
         a.k = sd;
         a.nq = B;
@@ -308,7 +315,7 @@ cudaError_t build_graph_with_scratch(int kind, const void* d_base, int64_t n, in
         a.bf_words = bf_words;
         a.bf_nhash = 4;
         a.n_multiprobe = 1;
-        search_warp_smem(kind, dim, a.cap, bf_words, &a);
+        search_warp_smem(kind, a.qdim, a.cap, bf_words, &a);
         e = cudaMemsetAsync(s.ctr, 0, 4, st);
         if (e == cudaSuccess) e = launch_search(kind, a, num_sms, st);
         if (e != cudaSuccess) break;

@@ -37,7 +37,7 @@ struct song_index {
     int64_t n = 0;
     int dim = 0;  // floats (L2) or u32 words (Hamming) per vector
     int ld = 0;   // padded row stride in elements (multiple of 4)
-    song::BaseRange range;  // integer range of the base (L2), for the exact-integer path
+    song::BaseRange range;  // integer range of the base (L2): decides on byte rows
     song_params p{};
     int device = 0;
     int num_sms = 0;
@@ -258,8 +258,7 @@ song_status create_common(int kind, const void* rows, int64_t n, int dim, const 
     // a pageable cudaMemcpy may return before its DMA lands: finish the legacy
     // stream before x->stream (non-blocking) reads the uploaded rows and adjacency
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-    if (e == cudaSuccess && kind == SONG_KIND_L2 && x->range.int_base && x->range.lo >= 0.0f &&
-        x->range.hi <= 255.0f && dim <= song::kU8MaxDim) {
+    if (e == cudaSuccess && kind == SONG_KIND_L2 && song::byte_rows(x->range, dim)) {
         x->u8_ld = song::u8_row_bytes(dim);
         e = cudaMalloc(&x->d_u8, (size_t)n * x->u8_ld);
         if (e == cudaSuccess)
@@ -393,11 +392,8 @@ song_status make_args(song_index* x, const void* d_q, int nq, int k, int ef, int
     a->bf_words = x->p.bf_words;
     a->bf_nhash = x->p.bf_nhash;
     a->n_multiprobe = x->p.n_multiprobe;
-    a->int_base = x->range.int_base;
-    a->base_min = x->range.lo;
-    a->base_max = x->range.hi;
     a->out_dist = d_dist;
-    a->qdim = x->dim;
+    a->qdim = x->kind == SONG_KIND_L2 ? x->ld : x->dim;
     a->u8 = x->d_u8;
     a->u8_ld = x->u8_ld;
     const int prec = opts ? opts->precision : SONG_PREC_FP32;
@@ -659,6 +655,10 @@ cudaError_t index_entry(song_index* x, const float* d_q, int qld, int nq, int32_
 int index_dim(const song_index* x) { return x ? x->dim : 0; }
 bool index_has_model(const song_index* x) { return x && x->has_model; }
 
+bool byte_rows(const BaseRange& r, int dim) {
+    return r.int_base && r.lo >= 0.0f && r.hi <= 255.0f && dim <= kU8MaxDim;
+}
+
 BaseRange scan_base_range(const float* rows, int64_t n, int dim) {
     BaseRange r;
     const int64_t total = n * (int64_t)dim;
@@ -793,6 +793,9 @@ song_status song_build_graph(int kind, const void* rows, int64_t n, int dim,
     if (e == cudaSuccess)
         e = cudaMemcpy2D(d_rows, row_bytes, rows, (size_t)dim * 4, (size_t)dim * 4, (size_t)n,
                          cudaMemcpyHostToDevice);
+    // a pageable copy may return before its DMA lands, and st does not wait for
+    // the legacy stream
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e == cudaSuccess)
         e = song::build_graph_device(kind, d_rows, n, dim, ld, *params, ratio, bfw, d_adj,
                                      sms, st, range);

@@ -38,8 +38,6 @@ struct SearchArgs {
     int q_off, rows_off, cd_off, ci_off, rd_off, ri_off, bl_off;  // per-warp carve-up, bytes
     int tm_cols;             // TMEM columns one CTA allocates (set by launch_search)
     int tm_warp_cols;        // TMEM columns of one warp's queue ids (set by launch_search)
-    int int_base;            // 1: every base value is an integer in [base_min, base_max]
-    float base_min, base_max;
     const uint8_t* u8;       // base values as bytes [n x u8_ld] when all are integers in [0, 255]
     int u8_ld;               // bytes per byte row (multiple of 16)
     // precision form (prec != SONG_PREC_FP32)
@@ -47,7 +45,7 @@ struct SearchArgs {
     const void* lowp;        // compressed rows [n x lowp_ld bytes]
     const float* scales;     // FP8: per-vector scale [n]
     int lowp_ld;             // bytes per compressed row (multiple of 128)
-    int qdim;                // floats of the query kept in shared memory (padded dim)
+    int qdim;                // floats of the query kept in shared memory (padded dim, at least ld)
     int rerank;              // 1: exact FP32 re-rank of the final results queue
     float* out_dist;         // [nq x k] distance of each output id (nullable)
     // learned entry / stop (lm: 0 off, 1 collect traces of the full search, 2 infer)
@@ -137,6 +135,8 @@ struct BaseRange {
     int int_base = 0;
     float lo = 0.0f, hi = 0.0f;
 };
+// Rows that may be kept as bytes (convert_rows_u8).
+bool byte_rows(const BaseRange& r, int dim);
 BaseRange scan_base_range(const float* rows, int64_t n, int dim);
 
 // Byte rows of integer-valued vectors: at most kU8MaxDim elements, each row

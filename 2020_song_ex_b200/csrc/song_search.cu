@@ -20,13 +20,13 @@
 //  * A row of up to 32 neighbours is handled at once, lane j = slot j, but
 //    the Bloom test of neighbour j sees the bits of neighbours < j exactly as
 //    bf_test/bf_set in j order do (bloomFilter.h:34-48): see bloom_chunk.
-//  * Distances follow warp_l2 (kernalGraph.h:157-170): lane l sums
-//    (q_i - b_i)^2 over i = l (mod 32) with FMA, then a butterfly
-//    transpose-reduce whose association is the reference's shfl_down tree.
-//    When every term and partial sum is an integer below 2^24 (integer
-//    vectors, the SIFT-shaped case) every order gives the same FP32 value,
-//    so those queries take a gather-only path instead: 8 lanes per row,
-//    16-byte loads, only the rows that passed the Bloom test.
+//  * Distances follow warp_l2 (kernalGraph.h:157-170): 32 partial sums of
+//    (q_i - b_i)^2 over i = l (mod 32) with FMA, then the reference's
+//    shfl_down tree.  Only the rows that passed the Bloom test are read, 8
+//    lanes per row with 16-byte loads, each lane holding four of the partial
+//    sums (l2_rows).  Integer vectors in [0, 255] (the SIFT-shaped case) are
+//    read as bytes instead: every order of exact integer sums gives the same
+//    FP32 value (l2_u8).
 //  * Pushes are applied in lane (= j) order; a push into a full queue only
 //    evicts when strictly closer than the current first maximum, and the
 //    maximum never grows while a queue is full, so lanes that lose against
@@ -562,119 +562,154 @@ __device__ __forceinline__ unsigned bloom_chunk(uint64_t* bloom, int nb, const B
     return __ballot_sync(FULL, (unc & ~cov) != 0u);
 }
 
-// Partial sum of lane `lane` for one row: sum over i = lane (mod 32) of
-// (q_i - b_i)^2 with FMA, in increasing i (warp_l2's per-lane loop).
-template <int NE>
-__device__ __forceinline__ float row_partial(const float* __restrict__ row, int dim,
-                                             const float (&qreg)[NE > 0 ? NE : 1],
-                                             const float* sq, int lane) {
-    float s = 0.0f;
-    if constexpr (NE > 0) {
-        float x[NE];
-#pragma unroll
-        for (int e = 0; e < NE; ++e) {
-            const int i = lane + 32 * e;
-            x[e] = i < dim ? ld_row(row + i) : 0.0f;
-        }
-#pragma unroll
-        for (int e = 0; e < NE; ++e) {
-            const int i = lane + 32 * e;
-            if (i < dim) {
-                const float t = qreg[e] - x[e];
-                s = fmaf(t, t, s);
-            }
-        }
+// Four floats of the query from element i on: 16 aligned bytes of shared
+// memory (QG = 0, zero padded to a multiple of 4), or the caller's own row in
+// global memory (QG = 1, any alignment, zero past dim).
+template <int QG>
+__device__ __forceinline__ float4 query4(const float* q, int i, int dim) {
+    if constexpr (QG) {
+        return make_float4(__ldg(q + i), i + 1 < dim ? __ldg(q + i + 1) : 0.0f,
+                           i + 2 < dim ? __ldg(q + i + 2) : 0.0f, i + 3 < dim ? __ldg(q + i + 3) : 0.0f);
     } else {
-        for (int i = lane; i < dim; i += 32) {
-            const float t = sq[i] - ld_row(row + i);
-            s = fmaf(t, t, s);
-        }
+        return *reinterpret_cast<const float4*>(q + i);
     }
-    return s;
 }
 
-// Squared L2 in the reference's exact order for the rows of the lanes in N;
-// lane j returns the distance of its own row.  Partial sums are combined by
-// a butterfly transpose-reduce: step w (16,8,4,2,1) pairs lanes l and l^w,
-// which is the reference tree's pairing of m and m+w.
-template <int NE>
-__device__ __forceinline__ float l2_exact(const float* __restrict__ base, int ld, int dim,
-                                          const float (&qreg)[NE > 0 ? NE : 1], const float* sq,
-                                          int nb, unsigned N, int lane) {
-    float v[16];
-    const bool up16 = lane & 16;
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const int id_lo = __shfl_sync(FULL, nb, r);
-        const int id_hi = __shfl_sync(FULL, nb, r + 16);
-        float s_lo = 0.0f, s_hi = 0.0f;
-        if ((N >> r) & 1u) s_lo = row_partial<NE>(base + (size_t)id_lo * ld, dim, qreg, sq, lane);
-        if ((N >> (r + 16)) & 1u) s_hi = row_partial<NE>(base + (size_t)id_hi * ld, dim, qreg, sq, lane);
-        const float send = up16 ? s_lo : s_hi;
-        const float keep = up16 ? s_hi : s_lo;
-        v[r] = keep + __shfl_xor_sync(FULL, send, 16);
-    }
-#pragma unroll
-    for (int w = 8; w >= 1; w >>= 1) {
-        const bool up = lane & w;
-#pragma unroll
-        for (int i = 0; i < w; ++i) {
-            const float send = up ? v[i] : v[i + w];
-            const float keep = up ? v[i + w] : v[i];
-            v[i] = keep + __shfl_xor_sync(FULL, send, w);
-        }
-    }
-    return v[0];
+// Elements of a row's float4 number c at or past dim := 0.
+__device__ __forceinline__ void drop_past(float4& x, int c, int dim) {
+    const int r = dim - 4 * c;
+    if (r < 4) x.w = 0.0f;
+    if (r < 3) x.z = 0.0f;
+    if (r < 2) x.y = 0.0f;
 }
 
-// Squared L2 when every partial sum is an exact integer (any order gives the
-// same FP32 value): only the rows of the lanes in N are gathered, 4 rows per
-// pass with 8 lanes per row and NV 16-byte loads per lane (dim = 32 * NV),
-// two passes in flight.  `rows` is a 32-entry per-warp shared list.
-template <int NV>
-__device__ __forceinline__ float l2_int(const float* __restrict__ base, int ld,
-                                        const float4 (&qv)[NV], int nb, unsigned N,
-                                        int* rows, int lane) {
+__device__ __forceinline__ void sq_diff4(const float4 q, const float4 x, float (&s)[4]) {
+    float t;
+    t = q.x - x.x; s[0] = fmaf(t, t, s[0]);
+    t = q.y - x.y; s[1] = fmaf(t, t, s[1]);
+    t = q.z - x.z; s[2] = fmaf(t, t, s[2]);
+    t = q.w - x.w; s[3] = fmaf(t, t, s[3]);
+}
+
+// Squared L2 in the reference's exact order (warp_l2, kernalGraph.h:157-170:
+// lane l sums i = l (mod 32) in increasing i with FMA, then a shfl_down tree
+// of 16, 8, 4, 2, 1) for the rows of the lanes in N; lane j gets its own
+// row's.  Only those rows are read, 4 per group of 8 lanes: lane t of a group
+// holds the partial sums of the reference's lanes 4t .. 4t + 3, since those
+// elements of every 32 are one 16-byte load, and the tree becomes shuffles
+// of 4, 2 and 1 between the lanes of a group (offsets 16, 8, 4) and of the
+// four sums among themselves (offsets 2, 1); a + b = b + a, so which side
+// keeps the sum does not matter.  The query is zero padded to 4 elements and
+// what a row holds past dim is dropped (a caller's rows may hold anything
+// there): a zero difference leaves every sum as it is.
+//
+// What bounds it is the wait for the rows, so the loads of up to 4 rows are
+// issued 8 per lane ahead of the sums (one round trip for dim <= 256), those
+// of up to 8 rows 4 + 4; 4 and 2 + 2 at 80 registers and 6 CTAs per SM
+// measured 10 % slower at 200 dimensions and 33 % at 960.  Reading each row
+// with 32 lanes of 4 bytes and reducing all 32 slots of the adjacency row in
+// unrolled code, as before, took 2-4 times the instructions and more code
+// than the instruction cache holds: 10,000 queries x 200 dimensions at ef 512
+// 36.3 -> 8.6 ms (200,000 nodes, 0.47 -> 2.0 TB/s of gathered rows), 1,000 x
+// 960 at ef 256 7.0 -> 2.5 ms, 10,000 x 24 at ef 128 4.4 -> 2.7 ms.
+template <int QG>
+__device__ __forceinline__ float l2_rows(const float* __restrict__ base, int ld, int dim,
+                                         const float* q, int nb, unsigned N, int* rows, int lane) {
     const bool mine = (N >> lane) & 1u;
     const int rank = __popc(N & lanemask_lt(lane));
     const int m = __popc(N);
     if (mine) rows[rank] = nb;
     __syncwarp();
     const int grp = lane >> 3, t = lane & 7;
+    const int nch = (dim + 3) >> 2;  // float4 per row
+    const bool ragged = dim & 3;
+    // loads in flight per lane and rows per pass; as few as can be where this is
+    // the rare path (QG), whose registers the byte rows' path would pay for
+    constexpr int U = QG ? 1 : 8, P = QG ? 4 : 8;
     float out = 0.0f;
-    for (int p0 = 0; p0 < m; p0 += 8) {
-        const int ra = p0 + grp, rb = p0 + 4 + grp;
-        float4 xa[NV], xb[NV];
+    for (int p0 = 0; p0 < m; p0 += P) {
+        const int ra = p0 + grp, rb = ra + 4;
         const bool va = ra < m, vb = rb < m;
         const float4* pa = reinterpret_cast<const float4*>(base + (size_t)(va ? rows[ra] : 0) * ld);
-        const float4* pb = reinterpret_cast<const float4*>(base + (size_t)(vb ? rows[rb] : 0) * ld);
+        float sa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float r;
+        if (P == 8 && m - p0 > 4) {
+            const float4* pb = reinterpret_cast<const float4*>(base + (size_t)(vb ? rows[rb] : 0) * ld);
+            float sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int c0 = t; c0 < nch; c0 += 4 * U) {
+                float4 xa[(U + 1) / 2], xb[(U + 1) / 2];
 #pragma unroll
-        for (int e = 0; e < NV; ++e) xa[e] = va ? ld_row(pa + t + 8 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int e = 0; e < U / 2; ++e) {
+                    const int c = c0 + 8 * e;
+                    const bool in = c < nch;
+                    xa[e] = (in && va) ? ld_row(pa + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    xb[e] = (in && vb) ? ld_row(pb + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                if (ragged) {
 #pragma unroll
-        for (int e = 0; e < NV; ++e) xb[e] = vb ? ld_row(pb + t + 8 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float sa = 0.0f, sb = 0.0f;
+                    for (int e = 0; e < U / 2; ++e) {
+                        drop_past(xa[e], c0 + 8 * e, dim);
+                        drop_past(xb[e], c0 + 8 * e, dim);
+                    }
+                }
 #pragma unroll
-        for (int e = 0; e < NV; ++e) {
-            float u;
-            u = qv[e].x - xa[e].x; sa = fmaf(u, u, sa);
-            u = qv[e].y - xa[e].y; sa = fmaf(u, u, sa);
-            u = qv[e].z - xa[e].z; sa = fmaf(u, u, sa);
-            u = qv[e].w - xa[e].w; sa = fmaf(u, u, sa);
-            u = qv[e].x - xb[e].x; sb = fmaf(u, u, sb);
-            u = qv[e].y - xb[e].y; sb = fmaf(u, u, sb);
-            u = qv[e].z - xb[e].z; sb = fmaf(u, u, sb);
-            u = qv[e].w - xb[e].w; sb = fmaf(u, u, sb);
+                for (int e = 0; e < U / 2; ++e) {
+                    const int c = c0 + 8 * e;
+                    if (c < nch) {
+                        const float4 qc = query4<QG>(q, 4 * c, dim);
+                        sq_diff4(qc, xa[e], sa);
+                        sq_diff4(qc, xb[e], sb);
+                    }
+                }
+            }
+            __syncwarp();
+            // offset 16 (lanes t, t ^ 4): lanes t < 4 keep row a, the others row b
+            const bool up = t & 4;
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float o = __shfl_xor_sync(FULL, up ? sa[i] : sb[i], 4);
+                v[i] = (up ? sb[i] : sa[i]) + o;
+            }
+            // offset 8 (t ^ 2) keeps sums {0, 1} or {2, 3}, offset 4 (t ^ 1) one of them
+            const bool u2 = t & 2, u1 = t & 1;
+            const float w0 = (u2 ? v[2] : v[0]) + __shfl_xor_sync(FULL, u2 ? v[0] : v[2], 2);
+            const float w1 = (u2 ? v[3] : v[1]) + __shfl_xor_sync(FULL, u2 ? v[1] : v[3], 2);
+            r = (u1 ? w1 : w0) + __shfl_xor_sync(FULL, u1 ? w0 : w1, 1);
+            r += __shfl_xor_sync(FULL, r, 2);  // offset 2: sums i and i ^ 2
+            r += __shfl_xor_sync(FULL, r, 1);  // offset 1: sums i and i ^ 1
+        } else {
+            for (int c0 = t; c0 < nch; c0 += 8 * U) {
+                float4 xa[U];
+#pragma unroll
+                for (int e = 0; e < U; ++e) {
+                    const int c = c0 + 8 * e;
+                    xa[e] = (c < nch && va) ? ld_row(pa + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                if (ragged) {
+#pragma unroll
+                    for (int e = 0; e < U; ++e) drop_past(xa[e], c0 + 8 * e, dim);
+                }
+#pragma unroll
+                for (int e = 0; e < U; ++e) {
+                    const int c = c0 + 8 * e;
+                    if (c < nch) sq_diff4(query4<QG>(q, 4 * c, dim), xa[e], sa);
+                }
+            }
+            __syncwarp();
+            // offset 16 keeps sums {0, 1} or {2, 3}, offset 8 one of them; offset 4
+            // adds the two halves of that sum; then offsets 2 and 1 as above
+            const bool u4 = t & 4, u2 = t & 2;
+            const float v0 = (u4 ? sa[2] : sa[0]) + __shfl_xor_sync(FULL, u4 ? sa[0] : sa[2], 4);
+            const float v1 = (u4 ? sa[3] : sa[1]) + __shfl_xor_sync(FULL, u4 ? sa[1] : sa[3], 4);
+            r = (u2 ? v1 : v0) + __shfl_xor_sync(FULL, u2 ? v0 : v1, 2);
+            r += __shfl_xor_sync(FULL, r, 1);  // offset 4
+            r += __shfl_xor_sync(FULL, r, 4);  // offset 2
+            r += __shfl_xor_sync(FULL, r, 2);  // offset 1
         }
-#pragma unroll
-        for (int w = 4; w >= 1; w >>= 1) {
-            sa += __shfl_xor_sync(FULL, sa, w);
-            sb += __shfl_xor_sync(FULL, sb, w);
-        }
-        // row of rank r sits in group r % 4 of pass r / 4
-        const float ga = __shfl_sync(FULL, sa, (rank & 3) << 3);
-        const float gb = __shfl_sync(FULL, sb, (rank & 3) << 3);
-        if (mine && (rank >> 2) == (p0 >> 2)) out = ga;
-        if (mine && (rank >> 2) == (p0 >> 2) + 1) out = gb;
+        // the row of rank r sits in group r % 4, the second rows in lanes 4 .. 7
+        const float g = __shfl_sync(FULL, r, ((rank & 3) << 3) | (P == 8 ? rank & 4 : 0));
+        if (mine && rank / P == p0 / P) out = g;
     }
     __syncwarp();
     return out;
@@ -1161,8 +1196,9 @@ __device__ __forceinline__ unsigned fkey(float x) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-// KIND 0 = L2 with NE query elements per lane (0: query in shared memory);
-// KIND 1 = Hamming with NE uint4 of code per row.  GPL: queue groups per lane.
+// KIND 0 = L2 (NE = 0: query in shared memory; NE < 0: byte rows of up to
+// -NE chunks of 16 bytes per lane); KIND 1 = Hamming with NE uint4 of code
+// per row.  GPL: queue groups per lane.
 // DT: SONG_PREC_FP32 (the plain, bit-exact search) or the precision form on
 // BF16 / FP8 rows (KIND 0, query in shared memory, FP32 re-rank at the end).
 // LM: 0 plain; 1 learning traces; 2 learned entry and stop; 3 learned entry
@@ -1198,90 +1234,21 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
     bc.wmask = (uint32_t)a.bf_words - 1u;
     bc.nhash = a.bf_nhash;
 
-    // Query in registers (and shared memory for the generic L2 path).
+    // The query: KIND 0 keeps it in shared memory (zero padded to qdim), but for
     // NE < 0 (byte-row instances, an index with byte rows, dim <= 32 * 4 * -NE):
-    // only the query's bytes stay in registers; a query that is not integral
-    // in [0, 255] takes the generic exact path reading its floats from global
+    // only the query's bytes, in registers; a query that is not integral in
+    // [0, 255] takes the exact float path reading its floats from global
     // memory.  Fewer live registers let more queries reside per SM.
     constexpr bool kU8 = KIND == 0 && NE < 0;
-    constexpr bool kIntPath = KIND == 0 && NE > 0 && DT == SONG_PREC_FP32;
-    constexpr int kNC = kU8 ? -NE : (NE >= 8 ? 2 : 1);  // 16-byte query chunks per lane on the byte-row path
-    float qreg[(KIND == 0 && NE > 0) ? NE : 1];
-    float4 qv[kIntPath ? NE : 1];
-    uint4 qb[(kIntPath || kU8) ? kNC : 1];
-    const float* sqg = sq;  // the query for the generic path (global memory in byte-row instances)
+    constexpr int kNC = kU8 ? -NE : 1;  // 16-byte query chunks per lane on the byte-row path
+    uint4 qb[kU8 ? kNC : 1];
+    const float* sqg = nullptr;  // byte-row instances: the query in global memory
     uint4 qcode[KIND == 1 ? NE : 1];
-    bool int_exact = false, u8_mode = false;
+    bool u8_mode = false;
     int qq = 0;
     if constexpr (KIND == 0) {
         const float* qg = reinterpret_cast<const float*>(a.queries) + (int64_t)qid * a.qld;
-        if constexpr (NE > 0) {
-            float lo = INFINITY, hi = -INFINITY;
-            bool integral = true;
-#pragma unroll
-            for (int e = 0; e < NE; ++e) {
-                const int i = lane + 32 * e;
-                qreg[e] = i < a.dim ? __ldcg(qg + i) : 0.0f;
-                if (i < a.dim) {
-                    lo = fminf(lo, qreg[e]);
-                    hi = fmaxf(hi, qreg[e]);
-                    integral &= qreg[e] == rintf(qreg[e]);
-                }
-            }
-            if (a.int_base && (a.dim == 32 * NE || a.u8 != nullptr)) {
-                // every |q_i - b_i| <= maxd; dim * maxd^2 < 2^24 keeps all sums exact
-                integral = __all_sync(FULL, integral);
-#pragma unroll
-                for (int w = 16; w >= 1; w >>= 1) {
-                    lo = fminf(lo, __shfl_xor_sync(FULL, lo, w));
-                    hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, w));
-                }
-                const double maxd = fmax((double)a.base_max - lo, (double)hi - a.base_min);
-                int_exact = integral && (double)a.dim * maxd * maxd < 16777216.0;
-                // byte rows (base in [0, 255]) and a query in [0, 255]: exact dp4a distances
-                u8_mode = kIntPath && int_exact && a.u8 != nullptr && lo >= 0.0f && hi <= 255.0f;
-                if (u8_mode) {
-                    int s2 = 0;
-#pragma unroll
-                    for (int e = 0; e < NE; ++e) {
-                        const int v = (int)qreg[e];  // zero beyond dim
-                        s2 += v * v;
-                    }
-                    qq = (int)__reduce_add_sync(FULL, (unsigned)s2);
-#pragma unroll
-                    for (int c = 0; c < kNC; ++c) {  // lane t of 8: bytes 16(t + 8c) .. +15
-                        const int e0 = 16 * ((lane & 7) + 8 * c);
-                        unsigned w4[4];
-#pragma unroll
-                        for (int wd = 0; wd < 4; ++wd) {
-                            unsigned wv = 0u;
-#pragma unroll
-                            for (int bt = 0; bt < 4; ++bt) {
-                                const int e = e0 + 4 * wd + bt;
-                                const unsigned bv = e < a.dim ? (unsigned)__ldcg(qg + e) : 0u;
-                                wv |= bv << (8 * bt);
-                            }
-                            w4[wd] = wv;
-                        }
-                        qb[c] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-                    }
-                } else if (int_exact && a.dim != 32 * NE) {
-                    int_exact = false;  // the float4 gather path needs dim == 32 * NE
-                }
-                if (int_exact && !u8_mode) {
-                    const float4* q4 = reinterpret_cast<const float4*>(qg);
-                    const bool aligned = ((reinterpret_cast<uintptr_t>(qg) & 15u) == 0);
-#pragma unroll
-                    for (int e = 0; e < NE; ++e) {
-                        const int f = (lane & 7) + 8 * e;
-                        qv[e] = aligned ? __ldcg(q4 + f)
-                                        : make_float4(__ldcg(qg + 4 * f), __ldcg(qg + 4 * f + 1),
-                                                      __ldcg(qg + 4 * f + 2), __ldcg(qg + 4 * f + 3));
-                    }
-                }
-            }
-        } else if constexpr (kU8) {
-            qreg[0] = 0.0f;
+        if constexpr (kU8) {
             sqg = qg;
             float lo = INFINITY, hi = -INFINITY;
             bool integral = true;
@@ -1323,7 +1290,6 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
                 }
             }
         } else {
-            qreg[0] = 0.0f;
             for (int i = lane; i < a.qdim; i += 32) sq[i] = i < a.dim ? __ldcg(qg + i) : 0.0f;
         }
     } else {
@@ -1345,15 +1311,11 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
             d = l2_lowp<DT>(a, sq, nb, N, rows, lane);
         } else if constexpr (KIND == 0) {
             const float* base = reinterpret_cast<const float*>(a.base);
-            if constexpr (kIntPath) {
+            if constexpr (kU8) {
                 if (u8_mode) d = l2_u8<kNC>(a.u8, a.u8_ld, a.u8_ld >> 4, qb, qq, nb, N, rows, lane);
-                else if (int_exact) d = l2_int<NE>(base, a.ld, qv, nb, N, rows, lane);
-                else d = l2_exact<NE>(base, a.ld, a.dim, qreg, sq, nb, N, lane);
-            } else if constexpr (kU8) {
-                if (u8_mode) d = l2_u8<kNC>(a.u8, a.u8_ld, a.u8_ld >> 4, qb, qq, nb, N, rows, lane);
-                else d = l2_exact<0>(base, a.ld, a.dim, qreg, sqg, nb, N, lane);
+                else d = l2_rows<1>(base, a.ld, a.dim, sqg, nb, N, rows, lane);
             } else {
-                d = l2_exact<NE>(base, a.ld, a.dim, qreg, sq, nb, N, lane);
+                d = l2_rows<0>(base, a.ld, a.dim, sq, nb, N, rows, lane);
             }
         } else {
             d = ham_lane<NE>(reinterpret_cast<const uint32_t*>(a.base), a.ld, a.dim, qcode, nb,
@@ -1769,14 +1731,9 @@ KernelSel pick_gpl(int kind, const SearchArgs& a) {
     if (kind == SONG_KIND_L2) {
         if (a.prec == SONG_PREC_BF16) return ksel<0, 0, GPL, SONG_PREC_BF16>();
         if (a.prec == SONG_PREC_FP8) return ksel<0, 0, GPL, SONG_PREC_FP8>();
-        if constexpr (GPL == 1) {  // an index with byte rows: the byte-row instances
-            if (a.u8 != nullptr && a.dim <= 128) return ksel<0, -1, 1, 0>();
-            if (a.u8 != nullptr && a.dim <= 256) return ksel<0, -2, 1, 0>();
-        }
-        if (a.dim <= 32) return ksel<0, 1, GPL, 0>();
-        if (a.dim <= 64) return ksel<0, 2, GPL, 0>();
-        if (a.dim <= 128) return ksel<0, 4, GPL, 0>();
-        if (a.dim <= 256) return ksel<0, 8, GPL, 0>();
+        // an index with byte rows: the byte-row instances
+        if (a.u8 != nullptr && a.dim <= 128) return ksel<0, -1, GPL, 0>();
+        if (a.u8 != nullptr && a.dim <= 256) return ksel<0, -2, GPL, 0>();
         return ksel<0, 0, GPL, 0>();
     }
     switch (a.ld) {
@@ -1835,7 +1792,6 @@ KernelSel pick_learned(const SearchArgs& a) {
     if (a.prec == SONG_PREC_BF16) return ksel<0, 0, 1, SONG_PREC_BF16, LM>();
     if (a.prec == SONG_PREC_FP8) return ksel<0, 0, 1, SONG_PREC_FP8, LM>();
     if (a.u8 != nullptr && a.dim <= 128) return ksel<0, -1, 1, 0, LM>();
-    if (a.dim <= 128 && a.dim > 64) return ksel<0, 4, 1, 0, LM>();
     return ksel<0, 0, 1, 0, LM>();
 }
 
@@ -1973,7 +1929,7 @@ cudaError_t launch_serve(const ServeArgs& s, int num_sms, int max_ctas, int rese
     const SearchArgs& a = s.base;
     if (a.prec == SONG_PREC_BF16) fn = serve_kernel<0, SONG_PREC_BF16>;
     else if (a.prec == SONG_PREC_FP8) fn = serve_kernel<0, SONG_PREC_FP8>;
-    else if (a.dim <= 128 && a.dim > 64) fn = serve_kernel<4, 0>;
+    else if (a.u8 != nullptr && a.dim <= 128) fn = serve_kernel<-1, 0>;
     else fn = serve_kernel<0, 0>;
     int dev = 0, optin = 0, smem_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -2011,9 +1967,8 @@ cudaError_t launch_serve(const ServeArgs& s, int num_sms, int max_ctas, int rese
     return cudaGetLastError();
 }
 
-cudaError_t launch_search(int kind, const SearchArgs& args, int num_sms, cudaStream_t stream) {
-    if (args.nq <= 0) return cudaSuccess;
-    KernelSel ks = pick_kernel(kind, args);
+static cudaError_t launch_instance(KernelSel ks, int kind, const SearchArgs& args, int num_sms,
+                                   cudaStream_t stream) {
     if (ks.fn == nullptr) return cudaErrorInvalidValue;
     if (args.trace == nullptr && ks.fn_nt != nullptr) {
         ks.fn = ks.fn_nt;
@@ -2065,6 +2020,11 @@ cudaError_t launch_search(int kind, const SearchArgs& args, int num_sms, cudaStr
             fn = ks.fn_tmd;
             tm_per_sm = p2;
         }
+        if (tm_per_sm < 1 && ks.query_smem && kind == SONG_KIND_L2 && a.prec == SONG_PREC_FP32 &&
+            args.dim <= kU8MaxDim) {
+            // four such warps leave no room for the query: read it from global memory
+            return launch_instance(ksel<0, -2, 1, 0>(), kind, args, num_sms, stream);
+        }
         if (tm_per_sm < 1) return cudaErrorInvalidConfiguration;
     } else {
         // Up to 8 warps per CTA while the CTA's shared memory stays within a
@@ -2104,6 +2064,11 @@ cudaError_t launch_search(int kind, const SearchArgs& args, int num_sms, cudaStr
     if (e != cudaSuccess) return e;
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError();
+}
+
+cudaError_t launch_search(int kind, const SearchArgs& args, int num_sms, cudaStream_t stream) {
+    if (args.nq <= 0) return cudaSuccess;
+    return launch_instance(pick_kernel(kind, args), kind, args, num_sms, stream);
 }
 
 }  // namespace song
