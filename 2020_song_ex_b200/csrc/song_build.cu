@@ -164,7 +164,7 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, 4, st);
     if (e == cudaSuccess && kind == SONG_KIND_L2 && byte_rows(range, dim)) {
         u8_ld = u8_row_bytes(dim);
-        e = cudaMalloc(&u8, (size_t)n * u8_ld);
+        e = device_alloc((void**)&u8, (size_t)n * u8_ld);
         if (e == cudaSuccess)
             e = convert_rows_u8(static_cast<const float*>(d_base), n, dim, ld, u8, u8_ld, st);
     }

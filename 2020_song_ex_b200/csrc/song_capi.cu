@@ -196,6 +196,7 @@ void free_index(song_index* x) {
     if (x->ev_d) cudaEventDestroy(x->ev_d);
     if (x->h_err) cudaFreeHost(x->h_err);
     if (x->stream) cudaStreamDestroy(x->stream);
+    song::trim_workspaces(x->device);
     cudaSetDevice(cur);
     delete x;
 }
@@ -225,8 +226,9 @@ song_status create_common(int kind, const void* rows, int64_t n, int dim, const 
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&x->num_sms, cudaDevAttrMultiProcessorCount, x->device);
     const size_t row_bytes = (size_t)x->ld * 4;
-    if (e == cudaSuccess) e = cudaMalloc(&x->d_base, (size_t)n * row_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&x->d_adj, (size_t)n * params->block_size * sizeof(int32_t));
+    if (e == cudaSuccess) e = song::device_alloc(&x->d_base, (size_t)n * row_bytes);
+    if (e == cudaSuccess)
+        e = song::device_alloc((void**)&x->d_adj, (size_t)n * params->block_size * sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMalloc(&x->d_counter, 2 * kCounterRing * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(x->d_counter, 0, 2 * kCounterRing * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMalloc(&x->d_err, 256);
@@ -260,7 +262,7 @@ song_status create_common(int kind, const void* rows, int64_t n, int dim, const 
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e == cudaSuccess && kind == SONG_KIND_L2 && song::byte_rows(x->range, dim)) {
         x->u8_ld = song::u8_row_bytes(dim);
-        e = cudaMalloc(&x->d_u8, (size_t)n * x->u8_ld);
+        e = song::device_alloc((void**)&x->d_u8, (size_t)n * x->u8_ld);
         if (e == cudaSuccess)
             e = song::convert_rows_u8((const float*)x->d_base, n, dim, x->ld, x->d_u8, x->u8_ld,
                                       x->stream);
@@ -786,8 +788,8 @@ song_status song_build_graph(int kind, const void* rows, int64_t n, int dim,
     int32_t* d_adj = nullptr;
     cudaStream_t st = nullptr;
     const size_t row_bytes = (size_t)ld * 4;
-    cudaError_t e = cudaMalloc(&d_rows, (size_t)n * row_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&d_adj, (size_t)n * params->block_size * 4);
+    cudaError_t e = song::device_alloc(&d_rows, (size_t)n * row_bytes);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&d_adj, (size_t)n * params->block_size * 4);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess && ld != dim) e = cudaMemset(d_rows, 0, (size_t)n * row_bytes);
     if (e == cudaSuccess)
@@ -822,7 +824,7 @@ song_status song_index_set_precision(song_index* x, int precision) {
     void** dst = precision == SONG_PREC_BF16 ? &x->d_bf16 : &x->d_fp8;
     cudaFree(*dst);
     *dst = nullptr;
-    SONG_CUDA(cudaMalloc(dst, (size_t)x->n * row_bytes), "compressed rows alloc");
+    SONG_CUDA(song::device_alloc(dst, (size_t)x->n * row_bytes), "compressed rows alloc");
     if (precision == SONG_PREC_FP8) {
         cudaFree(x->d_fp8_scale);
         x->d_fp8_scale = nullptr;

@@ -237,6 +237,11 @@ bool index_model_staged(const song_index* x);
 cudaError_t index_entry(song_index* x, const float* d_q, int qld, int nq, int32_t* d_ids,
                         float* d_d, cudaStream_t st, void* split_scratch, size_t split_bytes);
 
+// Workspace pool of calls without an index (song_gt.cu): give its kept memory
+// back; cudaMalloc that does so before it fails.
+void trim_workspaces(int dev);
+cudaError_t device_alloc(void** p, size_t bytes);
+
 // Records a failure message for song_last_error() on the calling thread.
 song_status set_error(song_status status, const char* message);
 

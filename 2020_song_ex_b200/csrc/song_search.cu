@@ -65,7 +65,6 @@ int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
 // Read-only loads of base rows (the read-only data path; an L1 no-allocate
 // variant measured slightly slower).
-__device__ __forceinline__ float ld_row(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float4 ld_row(const float4* p) { return __ldg(p); }
 __device__ __forceinline__ uint4 ld_row(const uint4* p) { return __ldg(p); }
 __device__ __forceinline__ unsigned lanemask_lt(int lane) { return (1u << lane) - 1u; }
