@@ -11,19 +11,41 @@
 // code is bit-identical to the reference's, including the signs of dot
 // products that land near zero.
 //
-// Layout of one CTA (128 threads): 64 vectors x 4 code words (128
-// hyperplanes).  Warp w owns code word blockIdx.y*4 + w; lane l owns vectors
-// l and l+32 and keeps all 32 dot products of its word for both, so the sign
-// bits pack in registers with no cross-lane step.  d advances in chunks of
-// 32: the chunk of the 64 vectors is staged in shared memory (padded rows:
-// lane l reads its own vector without bank conflicts) and the chunk of the
-// 128 hyperplanes is staged transposed (d-major, float4 groups swizzled by d)
-// so that the 32 hyperplanes of a word are read as 8 broadcast float4 loads.
-// Work is n * hash_bits * dim multiply-add pairs on the CUDA cores; R
-// (hash_bits * dim * 4 bytes) stays in L2.
+// Only the sign of that sum is wanted, so the tensor cores decide most bits
+// and the sequential sum only those near zero.  x = xh + xl and r = rh + rl
+// are split into BF16 parts; xh.rh and xh.rl + xl.rh are accumulated in two
+// FP32 accumulators, and their sum m differs from the reference's sum by less
+// than error_factor(dim) * |x| |r| (see there).  A bit with |m| above that
+// bound has the sign of m; the others (about one in 1,300 at 256 dimensions
+// of Gaussian data) are summed as above.  Every comparison with a NaN, an
+// overflow or a norm near the underflow range counts as "near zero", and if a
+// bounded wait gives up the CTA sums all of its remaining bits that way.
+//
+// One CTA takes 128 hyperplanes (4 code words), their BF16 parts resident in
+// shared memory up to 288 dimensions, and walks over tiles of 128 vectors;
+// the CTAs of the other words walk the same tiles at the same time, so x is
+// read from HBM once.  Warps have fixed roles:
+//   8 converters load chunks of 128 vectors x 32 dimensions (two chunks
+//     ahead in registers), split them into the tensor cores' operand layout in a
+//     ring of stages, and sum the squares for the bound;
+//   1 thread issues tcgen05.mma kind::f16 (M = N = 128, K = 16);
+//   2 sets of 4 epilogue warps, one per accumulator buffer, turn signs into
+//     code words with two funnel shifts per bit, free the buffer and then sum
+//     the near-zero bits of their tile, one per lane, under the next tile's
+//     products.
+// The floor is 3 products per multiply of the projection on the tensor cores
+// (0.14 ms for 290,000 x 256 -> 512 bits) or one pass over x (0.05 ms).  The
+// sums of all bits on the CUDA cores, 255 registers per thread and 8 warps per
+// SM, took 3.81 ms; this takes 0.47 ms (50,000 x 960 -> 1,024 bits 4.93 -> 1.13
+// ms, 1,000 x 256 -> 512 bits 41 -> 23 us).  What bounds it now is the
+// converters' loads of x: without products 0.41 ms, without near-zero sums
+// 0.43 ms.
 #include <cuda_runtime.h>
+#include <cuda_bf16.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <cstdint>
 #include <cstdio>
 #include <random>
@@ -38,91 +60,492 @@ extern std::atomic<int64_t> g_launches;
 
 namespace {
 
-constexpr int kTV = 64;     // vectors per CTA
-constexpr int kWords = 4;   // code words per CTA (one per warp)
-constexpr int kRows = kWords * 32;
-constexpr int kDC = 32;     // d per staged chunk
+constexpr unsigned FULL = 0xffffffffu;
+constexpr int kTV = 128;              // vectors per tile (MMA M, TMEM lanes)
+constexpr int kTB = 128;              // hyperplanes per CTA (MMA N)
+constexpr int kWords = kTB / 32;      // code words per CTA
+constexpr int kDC = 32;               // dimensions per chunk
+constexpr int kBlock = 128 * kDC * 2; // bytes of one 128 x 32 BF16 block
+constexpr int kResChunks = 9;         // resident hyperplanes: at most 9 chunks (288 dimensions)
+constexpr int kStagesRes = 4, kStagesStream = 6;
+constexpr int kThrSlots = 8;          // the converters run at most 8 tiles ahead of the epilogue: the
+                                      // ring's chunks and 2 tiles in the accumulators
+constexpr int kEpi = 8, kConv = 8;    // epilogue and converter warps
+constexpr int kThreads = 32 * (kEpi + 1 + kConv);
+constexpr int kItems = 128;           // near-zero bits a warp collects before it sums them
+constexpr long long kWaitCycles = 4000000000LL;  // about 2 s
 
-// Position of hyperplane `row` at chunk offset d in the transposed R tile:
-// float4 group (row / 4) is XOR-swizzled by d so that the transposing stores
-// of one warp (32 consecutive d, one row) spread over 8 banks.
-__device__ __forceinline__ int rs_pos(int d, int row) {
-    return d * kRows + ((((row >> 2) ^ d) & 31) << 2) + (row & 3);
+// Bound on |m - s| / (|x| |r|), with S = sum |x_i r_i| <= |x| |r|, u = 2^-24:
+//  * x - xh - xl is at most 2^-18 |x| (two roundings to 8 bits), so the
+//    products left out, xl.rl and the two remainders, are below 3.1 * 2^-18 S;
+//  * each tcgen05.mma adds 16 exact products and the accumulator, every one
+//    of them off by at most 2^-23 of the largest when they are aligned: 17 *
+//    2^-23 S per instruction, dim / 16 of them for xh.rh; the other
+//    accumulator holds terms 2^-8 as large (twice as many instructions);
+//  * the reference's sum itself: dim products and sums, below (dim + 1) u S,
+//    and the final m = main + cross below 2 u S.
+// The norms are FP32 sums of squares: 2^-10 covers their rounding.
+__host__ __device__ inline float error_factor(int dim) {
+    const float steps = (float)((dim + 15) / 16);
+    return (3.1f / 262144.0f + steps * (17.0f / 8388608.0f) * (1.0f + 2.0f / 256.0f) +
+            ((float)dim + 4.0f) / 16777216.0f) * (1.0f + 1.0f / 1024.0f);
 }
 
-__global__ void __launch_bounds__(128) bithash_kernel(const float* __restrict__ R, int dim,
-                                                      int words, const float* __restrict__ x,
-                                                      int64_t n, int64_t ldx,
-                                                      uint32_t* __restrict__ codes, int64_t ldc) {
-    __shared__ __align__(16) float xs[kTV][kDC + 1];
-    __shared__ __align__(16) float rs[kDC * kRows];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int64_t v0 = (int64_t)blockIdx.x * kTV;
-    const int w0 = blockIdx.y * kWords;
-    const int row0 = w0 * 32;
-    const int rows_here = min(kRows, words * 32 - row0);
-    const int my_word = w0 + warp;
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
 
-    float acc0[32], acc1[32];
-#pragma unroll
-    for (int b = 0; b < 32; ++b) {
-        acc0[b] = 0.0f;
-        acc1[b] = 0.0f;
+// Waits for the phase of parity `parity`; false after about 2 s, or as soon
+// as another warp has given up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+    const long long t0 = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if (*abort) return false;
+        if (clock64() - t0 > kWaitCycles) {
+            *abort = 1;
+            return false;
+        }
     }
+}
 
-    for (int d0 = 0; d0 < dim; d0 += kDC) {
-        const int cl = min(kDC, dim - d0);
-        __syncthreads();  // the previous chunk is consumed
-        // vectors: 64 x 32 floats, coalesced along d
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_addr(bar)) : "memory");
+}
+
+// Shared-memory matrix descriptor (tcgen05): start, leading and stride byte
+// offsets in 16-byte units, descriptor version 1, no swizzle.
+__device__ __forceinline__ uint64_t umma_desc(uint32_t start) {
+    return (uint64_t)((start >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) |
+           ((uint64_t)(512u >> 4) << 32) | (1ull << 46);
+}
+
+// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
+// K-major, N = 128, M = 128.
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTB >> 3) << 17) |
+                            ((uint32_t)(kTV >> 4) << 24);
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        :: "r"(tmem), "l"(ad), "l"(bd), "r"(kIdesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                 :: "r"(smem_addr(bar)) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait16(uint32_t (&a)[16], uint32_t (&b)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+        : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]),
+          "+r"(a[7]), "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]),
+          "+r"(a[14]), "+r"(a[15])
+        :: "memory");
 #pragma unroll
-        for (int i = 0; i < (kTV * kDC) / 128; ++i) {
-            const int idx = i * 128 + t;
-            const int v = idx >> 5, d = idx & 31;
-            const int64_t gv = v0 + v;
-            float val = 0.0f;
-            if (gv < n && d < cl) val = __ldg(x + gv * ldx + d0 + d);
-            xs[v][d] = val;
+    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(b[i]));
+}
+
+// 128 rows of FP32: the vectors of a tile or the hyperplanes of a CTA.
+struct Rows {
+    const float* p;   // row 0
+    int64_t ld;
+    int64_t count;    // rows that exist; the others read as zero
+    int dim;
+    bool vec;         // rows start on 16 bytes
+};
+
+// This lane's 8 elements of a chunk of 8 rows x 32 dimensions: row
+// (lane >> 1) & 7, dimensions 4 (lane & 1) + 8 (lane >> 4) + 16 h + 0 .. 3 for
+// h = 0, 1 (zero past the last row and dimension).  A load then takes whole
+// 32-byte sectors and a store to the operand layout 128 bytes of banks in a
+// row; with 4 lanes per row side by side 70 % of the shared-memory accesses
+// were bank conflicts and every sector was fetched twice.
+__device__ __forceinline__ int lane_row(int lane) { return (lane >> 1) & 7; }
+__device__ __forceinline__ int lane_dim(int lane) { return 4 * (lane & 1) + 8 * (lane >> 4); }
+__device__ __forceinline__ void load8(const Rows& s, int64_t r, int k0, float (&v)[8]) {
+    const float* p = s.p + r * s.ld + k0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (r < s.count && s.vec && k0 + 16 * h + 4 <= s.dim) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(p + 16 * h));
+            v[4 * h + 0] = a.x;
+            v[4 * h + 1] = a.y;
+            v[4 * h + 2] = a.z;
+            v[4 * h + 3] = a.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                v[4 * h + e] = (r < s.count && k0 + 16 * h + e < s.dim) ? __ldg(p + 16 * h + e) : 0.0f;
         }
-        // hyperplanes: 128 x 32 floats, coalesced along d, stored transposed
+    }
+}
+
+// Their BF16 hi and lo parts into the operand blocks at hi and hi + lo_off
+// (r8: group of 8 rows): K-major, no swizzle, 8 x 16-byte core matrices 128 B
+// apart along K, groups of 8 rows 512 B apart.
+__device__ __forceinline__ void store_split(unsigned char* hi, uint32_t lo_off, int r8, int lane, const float (&v)[8]) {
+    unsigned char* o = hi + r8 * 512 + (lane >> 4) * 128 + lane_row(lane) * 16 + (lane & 1) * 8;
 #pragma unroll
-        for (int i = 0; i < (kRows * kDC) / 128; ++i) {
-            const int idx = i * 128 + t;
-            const int row = idx >> 5, d = idx & 31;
-            float val = 0.0f;
-            if (row < rows_here && d < cl) val = __ldg(R + (int64_t)(row0 + row) * dim + d0 + d);
-            rs[rs_pos(d, row)] = val;
+    for (int h = 0; h < 2; ++h) {
+        __align__(8) __nv_bfloat162 a[2], b[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float x = v[4 * h + 2 * e], y = v[4 * h + 2 * e + 1];
+            a[e] = __floats2bfloat162_rn(x, y);
+            const float2 f = __bfloat1622float2(a[e]);
+            b[e] = __floats2bfloat162_rn(x - f.x, y - f.y);
         }
-        __syncthreads();
-        if (my_word < words) {
-            for (int d = 0; d < cl; ++d) {
-                const float xa = xs[lane][d];
-                const float xb = xs[lane + 32][d];
-                const float* rrow = rs + d * kRows;
+        *reinterpret_cast<uint2*>(o + h * 256) = *reinterpret_cast<const uint2*>(a);
+        *reinterpret_cast<uint2*>(o + h * 256 + lo_off) = *reinterpret_cast<const uint2*>(b);
+    }
+}
+
+// The reference's sum: a rounded product, then a rounded sum, in increasing d.
+__device__ __noinline__ float dot_seq(const float* __restrict__ r, const float* __restrict__ x, int dim, bool vec) {
+    float s = 0.0f;
+    int d = 0;
+    if (vec) {
+#pragma unroll 8
+        for (; d + 4 <= dim; d += 4) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(r + d));
+            const float4 b = __ldg(reinterpret_cast<const float4*>(x + d));
+            s = __fadd_rn(s, __fmul_rn(a.x, b.x));
+            s = __fadd_rn(s, __fmul_rn(a.y, b.y));
+            s = __fadd_rn(s, __fmul_rn(a.z, b.z));
+            s = __fadd_rn(s, __fmul_rn(a.w, b.w));
+        }
+    }
+#pragma unroll 4
+    for (; d < dim; ++d) s = __fadd_rn(s, __fmul_rn(__ldg(r + d), __ldg(x + d)));
+    return s;
+}
+
+struct BhArgs {
+    Rows R;           // all hyperplanes
+    Rows x;           // all vectors
+    uint32_t* codes;
+    int64_t ldc;
+    int words;        // code words per vector
+    int groups;       // CTAs side by side: ceil(words / kWords)
+    int per_group;    // CTAs of one group of words
+    int64_t tiles;    // tiles of 128 vectors
+    int nch;
+    float factor;     // error_factor(dim)
+};
+
+template <bool RES>
+__global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
+    constexpr int kStages = RES ? kStagesRes : kStagesStream;
+    constexpr uint32_t kStageBytes = (RES ? 2 : 4) * kBlock;  // xh, xl (, rh, rl)
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bar_full[kStages], bar_empty[kStages], bar_accf[2], bar_acce[2], bar_drain;
+    __shared__ float thr_s[kThrSlots][kTV];
+    __shared__ uint16_t item_s[kEpi][kItems];
+    __shared__ uint32_t fix_s[kEpi][32 * kWords];
+    __shared__ uint32_t tslot;
+    __shared__ unsigned rn2_s;  // largest squared norm of the CTA's hyperplanes (ordered bits)
+    __shared__ volatile int abort_flag, never;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    unsigned char* r_blocks = smem;                                       // RES: [hi, lo][nch][kBlock]
+    unsigned char* ring = smem + (RES ? (size_t)2 * a.nch * kBlock : 0);
+    const uint32_t r_lo = (uint32_t)a.nch * kBlock;
+
+    const int group = blockIdx.x % a.groups;
+    const int64_t first = blockIdx.x / a.groups;
+    const int64_t mytiles = first < a.tiles ? (a.tiles - first + a.per_group - 1) / a.per_group : 0;
+    Rows R = a.R;
+    R.p += (int64_t)group * kTB * R.ld;
+    R.count = min((int64_t)kTB, R.count - (int64_t)group * kTB);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(smem_addr(&tslot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&bar_full[s], kConv);
+            mbar_init(&bar_empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&bar_accf[b], 1);
+            mbar_init(&bar_acce[b], 4);
+        }
+        mbar_init(&bar_drain, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        rn2_s = 0u;
+        abort_flag = 0;
+        never = 0;
+    }
+    __syncthreads();
+    // the hyperplanes' norms and (RES) operand blocks: a warp per 8 of them
+    const int kd = lane_dim(lane);
+    {
+        float rn2 = 0.0f;
+        bool bad = false;
+        for (int r8 = warp; r8 < kTB / 8; r8 += kThreads / 32) {
+            const int r = r8 * 8 + lane_row(lane);
+            float q = 0.0f;
+            for (int c = 0; c < a.nch; ++c) {
+                float v[8];
+                load8(R, r, c * kDC + kd, v);
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int grp = warp * 8 + c;  // float4 group of hyperplanes 4*grp .. 4*grp+3
-                    const float4 r = *reinterpret_cast<const float4*>(rrow + (((grp ^ d) & 31) << 2));
-                    const float rv[4] = {r.x, r.y, r.z, r.w};
+                for (int e = 0; e < 8; ++e) q = fmaf(v[e], v[e], q);
+                if constexpr (RES) store_split(r_blocks + (size_t)c * kBlock, r_lo, r8, lane, v);
+            }
+            q += __shfl_xor_sync(FULL, q, 1);
+            q += __shfl_xor_sync(FULL, q, 16);
+            // near underflow the bound does not hold: none then (infinite)
+            if (r < R.count && !(q >= 1e-30f)) bad = true;
+            rn2 = fmaxf(rn2, q);
+        }
+        if (bad) rn2 = INFINITY;
+        atomicMax(&rn2_s, __float_as_uint(rn2));
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tslot;
+
+    if (warp > kEpi) {
+        // ---- converters ----
+        const int w = warp - kEpi - 1;
+        const float rbound = a.factor * sqrtf(__uint_as_float(rn2_s));
+        constexpr int kT = RES ? 2 : 4;  // 8 vectors each, then (streamed) 8 hyperplanes each
+        const int r0 = w * 8 + lane_row(lane);
+        const int64_t total = mytiles * a.nch;
+        int64_t fv0 = first * kTV;  // next chunk to load: first vector of its tile, chunk
+        int fc = 0;
+        auto fetch = [&](float (&d)[kT][8]) {
+            load8(a.x, fv0 + r0, fc * kDC + kd, d[0]);
+            load8(a.x, fv0 + r0 + 64, fc * kDC + kd, d[1]);
+            if constexpr (!RES) {
+                load8(R, r0, fc * kDC + kd, d[2]);
+                load8(R, r0 + 64, fc * kDC + kd, d[3]);
+            }
+            if (++fc == a.nch) {
+                fc = 0;
+                fv0 += (int64_t)a.per_group * kTV;
+            }
+        };
+        int s = 0, c = 0, slot = 0;
+        uint32_t parity = 1;  // the first round of the ring passes at once
+        float q0 = 0.0f, q1 = 0.0f;
+        unsigned any0 = 0u, any1 = 0u;
+        auto chunk = [&](float (&v)[kT][8], bool more) {
+            if (!__all_sync(FULL, mbar_wait(smem_addr(&bar_empty[s]), parity, &abort_flag))) return false;
+            unsigned char* st = ring + (size_t)s * kStageBytes;
+            store_split(st, kBlock, w, lane, v[0]);
+            store_split(st, kBlock, w + 8, lane, v[1]);
+            if constexpr (!RES) {
+                store_split(st + 2 * kBlock, kBlock, w, lane, v[2]);
+                store_split(st + 2 * kBlock, kBlock, w + 8, lane, v[3]);
+            }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int b = 4 * c + e;
-                        acc0[b] = __fadd_rn(acc0[b], __fmul_rn(rv[e], xa));
-                        acc1[b] = __fadd_rn(acc1[b], __fmul_rn(rv[e], xb));
+            for (int e = 0; e < 8; ++e) {
+                q0 = fmaf(v[0][e], v[0][e], q0);
+                q1 = fmaf(v[1][e], v[1][e], q1);
+                any0 |= __float_as_uint(v[0][e]) << 1;
+                any1 |= __float_as_uint(v[1][e]) << 1;
+            }
+            if (more) fetch(v);
+            if (++c == a.nch) {
+                c = 0;
+#pragma unroll
+                for (int o = 1; o <= 16; o <<= 4) {
+                    q0 += __shfl_xor_sync(FULL, q0, o);
+                    q1 += __shfl_xor_sync(FULL, q1, o);
+                    any0 |= __shfl_xor_sync(FULL, any0, o);
+                    any1 |= __shfl_xor_sync(FULL, any1, o);
+                }
+                // a zero vector's sums are zero (every bit certain: 0 > -1, clear); a norm
+                // near underflow has no bound
+                if ((lane & 17) == 0) {
+                    thr_s[slot][r0] = any0 == 0u ? -1.0f : (q0 >= 1e-30f ? rbound * sqrtf(q0) : INFINITY);
+                    thr_s[slot][r0 + 64] = any1 == 0u ? -1.0f : (q1 >= 1e-30f ? rbound * sqrtf(q1) : INFINITY);
+                }
+                slot = (slot + 1) % kThrSlots;
+                q0 = q1 = 0.0f;
+                any0 = any1 = 0u;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_full[s]);
+            if (++s == kStages) {
+                s = 0;
+                parity ^= 1u;
+            }
+            return true;
+        };
+        float va[kT][8], vb[kT][8];  // the next two chunks
+        if (total > 0) fetch(va);
+        if (total > 1) fetch(vb);
+        for (int64_t k = 0; k < total; k += 2) {
+            if (!chunk(va, k + 2 < total)) break;
+            if (k + 1 < total && !chunk(vb, k + 3 < total)) break;
+        }
+    } else if (warp == kEpi) {
+        // ---- MMA issuer ----
+        if (lane == 0) {
+            int s = 0;
+            uint32_t parity = 0;
+            bool ok = true;
+            const uint32_t ring_addr = smem_addr(ring);
+            const uint64_t r_desc = umma_desc(smem_addr(r_blocks));
+            for (int64_t i = 0; i < mytiles && ok; ++i) {
+                const int b = (int)(i & 1);
+                if (i >= 2 && !mbar_wait(smem_addr(&bar_acce[b]), (uint32_t)(((i >> 1) - 1) & 1), &abort_flag)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t main = tmem + (uint32_t)(b * 2 * kTB), cross = main + kTB;
+                for (int c = 0; c < a.nch; ++c) {
+                    ok = mbar_wait(smem_addr(&bar_full[s]), parity, &abort_flag);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t xh = umma_desc(ring_addr + (uint32_t)s * kStageBytes), xl = xh + kBlock / 16;
+                    const uint64_t rh = RES ? r_desc + (uint64_t)(c * (kBlock / 16)) : xl + kBlock / 16;
+                    const uint64_t rl = RES ? rh + r_lo / 16 : rh + kBlock / 16;
+#pragma unroll
+                    for (int ks = 0; ks < kDC / 16; ++ks) {
+                        const uint32_t acc = (c | ks) ? 1u : 0u;
+                        mma_bf16(main, xh + ks * 16, rh + ks * 16, acc);
+                        mma_bf16(cross, xh + ks * 16, rl + ks * 16, acc);
+                        mma_bf16(cross, xl + ks * 16, rh + ks * 16, 1u);
+                    }
+                    mma_commit(&bar_empty[s]);  // the stage is free once these MMAs ran
+                    if (++s == kStages) {
+                        s = 0;
+                        parity ^= 1u;
                     }
                 }
+                if (ok) mma_commit(&bar_accf[b]);
+            }
+            // every MMA issued has completed before the memory goes away
+            mma_commit(&bar_drain);
+            mbar_wait(smem_addr(&bar_drain), 0u, &never);
+        }
+    } else {
+        // ---- epilogue: set b reads accumulator buffer b; thread = vector = TMEM lane ----
+        const int b = warp >> 2;
+        const int row = (warp & 3) * 32 + lane;
+        const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(b * 2 * kTB);
+        const bool vec = a.x.vec && a.R.vec;
+        bool ok = true;
+        for (int64_t i = b; i < mytiles; i += 2) {
+            const int64_t v0 = (first + i * a.per_group) * kTV;
+            const int64_t v = v0 + row;
+            uint32_t word[kWords], unc[kWords];
+            if (ok) ok = __all_sync(FULL, mbar_wait(smem_addr(&bar_accf[b]), (uint32_t)((i >> 1) & 1), &abort_flag));
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const float thr = thr_s[i % kThrSlots][row];
+#pragma unroll
+                for (int w = 0; w < kWords; ++w) {
+                    uint32_t bits = 0u, sure = 0u;
+#pragma unroll
+                    for (int h = 1; h >= 0; --h) {
+                        uint32_t m[16], x[16];
+                        tmem_ld16(acc + (uint32_t)(w * 32 + h * 16), m);
+                        tmem_ld16(acc + (uint32_t)(kTB + w * 32 + h * 16), x);
+                        tmem_wait16(m, x);
+#pragma unroll
+                        for (int j = 15; j >= 0; --j) {  // bit j of the half: sign of 0 - sum, sign of bound - |sum|
+                            const float sum = __fadd_rn(__uint_as_float(m[j]), __uint_as_float(x[j]));
+                            bits = __funnelshift_l(__float_as_uint(__fsub_rn(0.0f, sum)), bits, 1);
+                            sure = __funnelshift_l(__float_as_uint(__fsub_rn(thr, fabsf(sum))), sure, 1);
+                        }
+                    }
+                    word[w] = bits;
+                    unc[w] = ~sure;
+                }
+                // the accumulator has been read: the MMAs may overwrite it
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_acce[b]);
+            } else {
+#pragma unroll
+                for (int w = 0; w < kWords; ++w) {
+                    word[w] = 0u;
+                    unc[w] = FULL;
+                }
+            }
+            const int nw = min(kWords, a.words - group * kWords);
+            int cnt = 0;
+#pragma unroll
+            for (int w = 0; w < kWords; ++w) {
+                if (v >= a.x.count || w >= nw) unc[w] = 0u;
+                cnt += __popc(unc[w]);
+            }
+            int before = cnt;  // inclusive prefix over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULL, before, o);
+                if (lane >= o) before += t;
+            }
+            const int total = __shfl_sync(FULL, before, 31);
+            before -= cnt;
+            if (total > kItems) {  // many (data made of near-zero sums): each lane sums its own
+#pragma unroll
+                for (int w = 0; w < kWords; ++w)
+                    while (unc[w]) {
+                        const int j = __ffs(unc[w]) - 1;
+                        unc[w] &= unc[w] - 1u;
+                        const float s = dot_seq(R.p + (int64_t)(w * 32 + j) * R.ld, a.x.p + v * a.x.ld, R.dim, vec);
+                        word[w] = (word[w] & ~(1u << j)) | ((s > 0.0f ? 1u : 0u) << j);
+                    }
+            } else if (total > 0) {  // few: spread over the lanes
+#pragma unroll
+                for (int w = 0; w < kWords; ++w) {
+                    fix_s[warp][lane * kWords + w] = word[w] & ~unc[w];
+                    for (unsigned m = unc[w]; m; m &= m - 1u)
+                        item_s[warp][before++] = (uint16_t)(lane * kTB + w * 32 + __ffs(m) - 1);
+                }
+                __syncwarp();
+                for (int t = lane; t < total; t += 32) {
+                    const int it = item_s[warp][t], l = it / kTB, j = it % kTB;
+                    const float s = dot_seq(R.p + (int64_t)j * R.ld,
+                                            a.x.p + (v0 + (warp & 3) * 32 + l) * a.x.ld, R.dim, vec);
+                    if (s > 0.0f) atomicOr(&fix_s[warp][l * kWords + (j >> 5)], 1u << (j & 31));
+                }
+                __syncwarp();
+#pragma unroll
+                for (int w = 0; w < kWords; ++w) word[w] = fix_s[warp][lane * kWords + w];
+                __syncwarp();
+            }
+            if (v < a.x.count) {
+                uint32_t* out = a.codes + v * a.ldc + group * kWords;
+#pragma unroll
+                for (int w = 0; w < kWords; ++w)
+                    if (w < nw) out[w] = word[w];
             }
         }
     }
-    if (my_word >= words) return;
-    uint32_t c0 = 0, c1 = 0;
-#pragma unroll
-    for (int b = 0; b < 32; ++b) {
-        c0 |= (acc0[b] > 0.0f ? 1u : 0u) << b;
-        c1 |= (acc1[b] > 0.0f ? 1u : 0u) << b;
-    }
-    const int64_t va = v0 + lane, vb = v0 + lane + 32;
-    if (va < n) codes[va * ldc + my_word] = c0;
-    if (vb < n) codes[vb * ldc + my_word] = c1;
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512) : "memory");
 }
 
 song_status fail(song_status s, const char* msg) { return song::set_error(s, msg); }
@@ -148,9 +571,27 @@ namespace song {
 cudaError_t launch_bithash(const float* d_R, int dim, int hash_bits, const float* d_x, int64_t n,
                            int64_t ldx, uint32_t* d_codes, int64_t ldc, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const int words = hash_bits / 32;
-    const dim3 grid((unsigned)((n + kTV - 1) / kTV), (unsigned)((words + kWords - 1) / kWords));
-    bithash_kernel<<<grid, 128, 0, st>>>(d_R, dim, words, d_x, n, ldx, d_codes, ldc);
+    int dev = 0, num_sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    BhArgs a;
+    a.R = Rows{d_R, dim, hash_bits, dim, (reinterpret_cast<uintptr_t>(d_R) & 15u) == 0 && dim % 4 == 0};
+    a.x = Rows{d_x, ldx, n, dim, (reinterpret_cast<uintptr_t>(d_x) & 15u) == 0 && ldx % 4 == 0};
+    a.codes = d_codes;
+    a.ldc = ldc;
+    a.words = hash_bits / 32;
+    a.groups = (a.words + kWords - 1) / kWords;
+    a.tiles = (n + kTV - 1) / kTV;
+    a.per_group = (int)std::min<int64_t>(std::max(1, num_sms / a.groups), a.tiles);
+    a.nch = (dim + kDC - 1) / kDC;
+    a.factor = error_factor(dim);
+    const bool res = a.nch <= kResChunks;
+    const size_t smem = res ? (size_t)(2 * a.nch + 2 * kStagesRes) * kBlock : (size_t)4 * kStagesStream * kBlock;
+    void (*kern)(const BhArgs) = res ? bithash_kernel<true> : bithash_kernel<false>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<(unsigned)(a.per_group * a.groups), kThreads, smem, st>>>(a);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError();
 }
@@ -180,7 +621,7 @@ song_status song_bithash_project_device(const float* d_R, int dim, int hash_bits
         return fail(SONG_ERR_INVALID_ARG, "R, x or codes is NULL");
     if (ldx < dim) return fail(SONG_ERR_INVALID_ARG, "ldx must be >= dim");
     if (ldc < hash_bits / 32) return fail(SONG_ERR_INVALID_ARG, "ldc must be >= hash_bits / 32");
-    if ((n + kTV - 1) / kTV > (int64_t)INT32_MAX)
+    if ((n + 63) / 64 > (int64_t)INT32_MAX)
         return fail(SONG_ERR_INVALID_ARG, "n too large for one launch");
     cudaError_t e = song::launch_bithash(d_R, dim, hash_bits, d_x, n, ldx, d_codes, ldc,
                                          (cudaStream_t)stream);
