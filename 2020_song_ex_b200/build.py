@@ -13,9 +13,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsong_b200.so")
-SOURCES = ["song_search.cu", "song_build.cu", "song_learn.cu", "song_capi.cu", "song_serve.cu",
-           "song_noalloc.cu", "song_bithash.cu", "song_entry.cu",
-           "song_graphsearch.cu", "song_gt.cu"]
+SOURCES = ["song_search_l2.cu", "song_search_learned.cu", "song_search_hamming.cu",
+           "song_search_lowp.cu", "song_search.cu", "song_build.cu", "song_learn.cu",
+           "song_capi.cu", "song_serve.cu", "song_noalloc.cu", "song_bithash.cu",
+           "song_entry.cu", "song_graphsearch.cu", "song_gt.cu"]
 NVCC = os.environ.get("NVCC", "nvcc")
 FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
