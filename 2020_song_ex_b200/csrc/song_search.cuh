@@ -57,9 +57,9 @@ using KernelFn = void (*)(const SearchArgs);
 struct KernelSel {
     KernelFn fn = nullptr;      // candidate ids in shared memory
     KernelFn fn_tmc = nullptr;  // tm only: the candidate ids in TMEM too
-    KernelFn fn_nt = nullptr;   // byte-row instances: fn and fn_tmc without the trace
+    KernelFn fn_tmd = nullptr;  // tm only, not all: result distances in TMEM too
+    KernelFn fn_nt = nullptr;   // the three without the trace, where they exist
     KernelFn fn_tmc_nt = nullptr;
-    KernelFn fn_tmd = nullptr;  // byte-row plain instances: result distances in TMEM too
     KernelFn fn_tmd_nt = nullptr;
     int tm = 0;                 // result ids in TMEM (the CTA allocates tensor memory)
     int qr = 0;                 // queues in registers: up to 32 * qr slots
@@ -1143,14 +1143,27 @@ __device__ __forceinline__ int finish(RQueue<R>& res, int k, int32_t* out, float
     return cnt;
 }
 
+// Place in shared memory of query element i for the compressed rows: lane t of
+// 8 reads the elements of row chunk t + 8 b (EPC of them) four at a time, so
+// the four's 8 places are side by side.  In element order the 8 lanes' reads
+// were 32 or 64 bytes apart, 2 and 4 bank conflicts each (4,000 queries x 960
+// dimensions, FP8, ef 384: 6.14 -> 5.91 ms).
+template <int DT>
+__device__ __forceinline__ int lowp_place(int i) {
+    constexpr int EPC = DT == SONG_PREC_BF16 ? 8 : 16;  // elements per 16-byte chunk
+    const int c = i / EPC, piece = (i % EPC) >> 2;
+    return ((c >> 3) * (EPC / 4) + piece) * 32 + (c & 7) * 4 + (i & 3);
+}
+
 // Accumulate (q - b)^2 over one 16-byte chunk of a compressed row: 8 BF16 or
-// 16 FP8 e4m3 values (times the row's scale), FP32 arithmetic.
+// 16 FP8 e4m3 values (times the row's scale), FP32 arithmetic.  qc: the
+// chunk's first four query elements, the next ones 32 floats on.
 template <int DT>
 __device__ __forceinline__ void chunk_l2(const uint4 x, const float* qc, float scale, float& acc) {
     const unsigned w[4] = {x.x, x.y, x.z, x.w};
     if constexpr (DT == SONG_PREC_BF16) {
         const float4 q0 = *reinterpret_cast<const float4*>(qc);
-        const float4 q1 = *reinterpret_cast<const float4*>(qc + 4);
+        const float4 q1 = *reinterpret_cast<const float4*>(qc + 32);
         const float q[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -1164,7 +1177,7 @@ __device__ __forceinline__ void chunk_l2(const uint4 x, const float* qc, float s
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float4 q = *reinterpret_cast<const float4*>(qc + 4 * i);
+            const float4 q = *reinterpret_cast<const float4*>(qc + 32 * i);
             const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[i] & 0xffffu), __NV_E4M3);
             const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[i] >> 16), __NV_E4M3);
             const float2 b01 = __half22float2(__half2(h01));
@@ -1190,6 +1203,7 @@ __device__ __forceinline__ float l2_lowp(const SearchArgs& a, const float* sq, i
     constexpr int EPC = DT == SONG_PREC_BF16 ? 8 : 16;  // elements per 16-byte chunk
     const int grp = lane >> 3, t = lane & 7;
     const int nchunk = a.lowp_ld >> 4;
+    const float* qt = sq + 4 * t;  // chunk t + 8 b of the query: 8 EPC b floats on
     const unsigned char* lp = reinterpret_cast<const unsigned char*>(a.lowp);
     float out = 0.0f;
     for (int p0 = 0; p0 < m; p0 += 8) {
@@ -1203,12 +1217,36 @@ __device__ __forceinline__ float l2_lowp(const SearchArgs& a, const float* sq, i
             sca = va ? __ldg(a.scales + ia) : 0.0f;
             scb = vb ? __ldg(a.scales + ib) : 0.0f;
         }
+        // rows are whole multiples of 8 chunks; loads in flight per lane: 4 of one
+        // row, or 2 of each of two rows
         float sa = 0.0f, sb = 0.0f;
-        for (int c = t; c < nchunk; c += 8) {
-            const uint4 xa = va ? ld_row(pa + c) : make_uint4(0u, 0u, 0u, 0u);
-            const uint4 xb = vb ? ld_row(pb + c) : make_uint4(0u, 0u, 0u, 0u);
-            chunk_l2<DT>(xa, sq + c * EPC, sca, sa);
-            chunk_l2<DT>(xb, sq + c * EPC, scb, sb);
+        if (m - p0 > 4) {
+            for (int c0 = t; c0 < nchunk; c0 += 16) {
+                uint4 xa[2], xb[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const bool in = c0 + 8 * e < nchunk;
+                    xa[e] = (in && va) ? ld_row(pa + c0 + 8 * e) : make_uint4(0u, 0u, 0u, 0u);
+                    xb[e] = (in && vb) ? ld_row(pb + c0 + 8 * e) : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (c0 + 8 * e < nchunk) {
+                        chunk_l2<DT>(xa[e], qt + (c0 - t + 8 * e) * EPC, sca, sa);
+                        chunk_l2<DT>(xb[e], qt + (c0 - t + 8 * e) * EPC, scb, sb);
+                    }
+                }
+            }
+        } else {
+            for (int c0 = t; c0 < nchunk; c0 += 32) {
+                uint4 xa[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    xa[e] = (c0 + 8 * e < nchunk && va) ? ld_row(pa + c0 + 8 * e) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c0 + 8 * e < nchunk) chunk_l2<DT>(xa[e], qt + (c0 - t + 8 * e) * EPC, sca, sa);
+            }
         }
 #pragma unroll
         for (int w = 4; w >= 1; w >>= 1) {
@@ -1222,6 +1260,41 @@ __device__ __forceinline__ float l2_lowp(const SearchArgs& a, const float* sq, i
     }
     __syncwarp();
     return out;
+}
+
+// Squared FP32 distance of the row `row` (nullptr: none) for each group of 8
+// lanes, summed per lane over every 8th float4 and then over the lanes: 8
+// loads in flight per lane, or the final re-rank (every entry of a queue) is
+// a chain of one load after the other (with the one-row pass of l2_lowp,
+// 4,000 queries x 960 dimensions at ef 384: FP8 7.48 -> 6.14 ms, BF16 9.38 ->
+// 6.94 ms).
+__device__ __forceinline__ float rerank_row(const float4* row, int nch, const float* sq, int lane) {
+    constexpr int U = 8;
+    const int t = lane & 7;
+    float acc = 0.0f;
+    for (int c0 = t; c0 < nch; c0 += 8 * U) {
+        float4 x[U];
+#pragma unroll
+        for (int e = 0; e < U; ++e)
+            x[e] = (row != nullptr && c0 + 8 * e < nch) ? ld_row(row + c0 + 8 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < U; ++e) {
+            if (c0 + 8 * e < nch) {
+                const float4 q = *reinterpret_cast<const float4*>(sq + 4 * (c0 + 8 * e));
+                float u = q.x - x[e].x;
+                acc = fmaf(u, u, acc);
+                u = q.y - x[e].y;
+                acc = fmaf(u, u, acc);
+                u = q.z - x[e].z;
+                acc = fmaf(u, u, acc);
+                u = q.w - x[e].w;
+                acc = fmaf(u, u, acc);
+            }
+        }
+    }
+#pragma unroll
+    for (int w = 4; w >= 1; w >>= 1) acc += __shfl_xor_sync(FULL, acc, w);
+    return acc;
 }
 
 // Precision form, final step: exact FP32 distances of every entry of the
@@ -1249,22 +1322,7 @@ __device__ __forceinline__ int rerank_finish(const SearchArgs& a, Queue<GPL, TM,
         } else {
             id = v ? res.id[r] : 0;
         }
-        const float4* row = reinterpret_cast<const float4*>(base + (size_t)id * a.ld);
-        float acc = 0.0f;
-        for (int c = t; c < nch; c += 8) {
-            const float4 x = v ? ld_row(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 q = *reinterpret_cast<const float4*>(sq + 4 * c);
-            float u = q.x - x.x;
-            acc = fmaf(u, u, acc);
-            u = q.y - x.y;
-            acc = fmaf(u, u, acc);
-            u = q.z - x.z;
-            acc = fmaf(u, u, acc);
-            u = q.w - x.w;
-            acc = fmaf(u, u, acc);
-        }
-#pragma unroll
-        for (int w = 4; w >= 1; w >>= 1) acc += __shfl_xor_sync(FULL, acc, w);
+        const float acc = rerank_row(v ? reinterpret_cast<const float4*>(base + (size_t)id * a.ld) : nullptr, nch, sq, lane);
         if (t == 0 && v) {
             rd[r] = acc;
             if constexpr (!TM) rid[r] = id;
@@ -1321,22 +1379,8 @@ __device__ __forceinline__ int rerank_finish(const SearchArgs& a, RQueue<R>& res
     const int grp = lane >> 3, t = lane & 7;
     for (int p0 = 0; p0 < m; p0 += 4) {
         const bool v = p0 + grp < m;
-        const float4* row = reinterpret_cast<const float4*>(base + (size_t)(v ? res.id[p0 + grp] : 0) * a.ld);
-        float acc = 0.0f;
-        for (int c = t; c < nch; c += 8) {
-            const float4 x = v ? ld_row(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 q = *reinterpret_cast<const float4*>(sq + 4 * c);
-            float u = q.x - x.x;
-            acc = fmaf(u, u, acc);
-            u = q.y - x.y;
-            acc = fmaf(u, u, acc);
-            u = q.z - x.z;
-            acc = fmaf(u, u, acc);
-            u = q.w - x.w;
-            acc = fmaf(u, u, acc);
-        }
-#pragma unroll
-        for (int w = 4; w >= 1; w >>= 1) acc += __shfl_xor_sync(FULL, acc, w);
+        const float4* row = v ? reinterpret_cast<const float4*>(base + (size_t)res.id[p0 + grp] * a.ld) : nullptr;
+        const float acc = rerank_row(row, nch, sq, lane);
         if (t == 0 && v) rd[p0 + grp] = acc;
     }
     __syncwarp();
@@ -1609,7 +1653,11 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
                 }
             }
         } else {
-            for (int i = lane; i < a.qdim; i += 32) sq[i] = i < a.dim ? __ldcg(qg + i) : 0.0f;
+            for (int i = lane; i < a.qdim; i += 32) {
+                const float v = i < a.dim ? __ldcg(qg + i) : 0.0f;
+                if constexpr (DT != SONG_PREC_FP32) sq[lowp_place<DT>(i)] = v;
+                else sq[i] = v;
+            }
         }
     } else {
         const uint32_t* qg = reinterpret_cast<const uint32_t*>(a.queries) + (int64_t)qid * a.qld;
@@ -1957,6 +2005,14 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
     // finished writes nothing until that launch is complete
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float* outd = a.out_dist ? a.out_dist + (int64_t)qid * a.k : nullptr;
+    if constexpr (DT != SONG_PREC_FP32) {
+        if (a.rerank) {  // the FP32 rows' distances read the query in element order
+            const float* qg = reinterpret_cast<const float*>(a.queries) + (int64_t)qid * a.qld;
+            __syncwarp();
+            for (int i = lane; i < a.qdim; i += 32) sq[i] = i < a.dim ? __ldcg(qg + i) : 0.0f;
+            __syncwarp();
+        }
+    }
     if constexpr (QR) {
         if (DT != SONG_PREC_FP32 && a.rerank)
             tr.result_count = rerank_finish(a, res, sq, a.out + (int64_t)qid * a.k, outd, lane,
@@ -2005,7 +2061,7 @@ struct KernelShape {
                             : (LM == 2 ? (NE < 0 ? 5 : 4) : (NE < 0 ? 6 : 5)))
                  : 1;
     // without the trace counters (TR = 0): one more CTA
-    static constexpr int kMinBlocksNT = GPL == 1 && NE < 0 ? kMinBlocks + 1 : kMinBlocks;
+    static constexpr int kMinBlocksNT = GPL == 1 && (NE < 0 || KIND == 1) ? kMinBlocks + 1 : kMinBlocks;
     // register queues: 96 registers (5 CTAs), without the trace counters 80 (6); float
     // rows keep 8 loads in flight and spilled at 96: 128 (4 CTAs), 15 % faster at 500
     // queries and 960 dimensions, the same at 10,000
@@ -2084,14 +2140,15 @@ KernelSel ksel() {
     KernelSel k;
     k.fn = search_kernel<KIND, NE, GPL, DT, LM, 0>;
     if constexpr (S::kTM) k.fn_tmc = search_kernel<KIND, NE, GPL, DT, LM, 1>;
-    if constexpr (NE < 0 && LM != 1) {  // trace-free copies of the hot instances
+    if constexpr ((NE < 0 || KIND == 1) && LM != 1) {  // trace-free copies where they fit one more CTA
         k.fn_nt = search_kernel<KIND, NE, GPL, DT, LM, 0, 0>;
         if constexpr (S::kTM) {
             k.fn_tmc_nt = search_kernel<KIND, NE, GPL, DT, LM, 1, 0>;
-            k.fn_tmd = search_kernel<KIND, NE, GPL, DT, LM, 1, 1, 1>;
             k.fn_tmd_nt = search_kernel<KIND, NE, GPL, DT, LM, 1, 0, 1>;
         }
     }
+    if constexpr (S::kTM && (NE < 0 || KIND == 1 || DT != SONG_PREC_FP32))
+        k.fn_tmd = search_kernel<KIND, NE, GPL, DT, LM, 1, 1, 1>;
     k.tm = S::kTM;
     k.threads = S::kThreads;
     k.query_smem = S::kQuerySmem;
@@ -2103,7 +2160,7 @@ KernelSel ksel_reg() {
     using S = KernelShape<KIND, NE, 1, DT, LM, QR>;
     KernelSel k;
     k.fn = search_kernel<KIND, NE, 1, DT, LM, 0, 1, 0, QR>;
-    if constexpr (NE < 0) k.fn_nt = search_kernel<KIND, NE, 1, DT, LM, 0, 0, 0, QR>;
+    if constexpr (NE < 0 || KIND == 1) k.fn_nt = search_kernel<KIND, NE, 1, DT, LM, 0, 0, 0, QR>;
     k.qr = QR;
     k.threads = S::kThreads;
     k.query_smem = S::kQuerySmem;
