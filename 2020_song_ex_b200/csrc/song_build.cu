@@ -127,7 +127,7 @@ __global__ void reverse_edges(const uint32_t* __restrict__ keys, const uint32_t*
 // ([n x ld], kind L2 or Hamming).  Stream-ordered; returns a CUDA error.
 cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim, int ld,
                                const song_params& p, int ratio, int bf_words, int32_t* d_adj,
-                               int num_sms, cudaStream_t st, BaseRange range) {
+                               int num_sms, cudaStream_t st) {
     if (ratio < 1) ratio = 32;
     const int bs = p.block_size, fd = p.fixed_degree, sd = p.search_degree;
     if (fd > 32 || fd > bs || sd < 1) return cudaErrorInvalidValue;
@@ -145,26 +145,33 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
     uint8_t* u8 = nullptr;  // byte copy of integer rows in [0, 255]: a quarter of the gathered bytes
     int u8_ld = 0;
     auto cleanup = [&]() {
-        cudaFree(d_fwd); cudaFree(k0); cudaFree(k1); cudaFree(v0); cudaFree(v1);
-        cudaFree(ctr); cudaFree(err); cudaFree(tmp); cudaFree(u8);
+        for (void* q : {(void*)d_fwd, (void*)k0, (void*)k1, (void*)v0, (void*)v1, (void*)ctr, tmp, (void*)u8})
+            if (q != nullptr) cudaFreeAsync(q, st);
     };
-    if ((e = cudaMalloc(&d_fwd, maxB * sd * sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMalloc(&k0, maxE * 4)) != cudaSuccess || (e = cudaMalloc(&k1, maxE * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&v0, maxE * 4)) != cudaSuccess || (e = cudaMalloc(&v1, maxE * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&ctr, 4)) != cudaSuccess || (e = cudaMalloc(&err, 4)) != cudaSuccess) {
+    // ctr: work counter, error word, scan results
+    if ((e = workspace_alloc((void**)&d_fwd, maxB * sd * sizeof(int32_t), st)) != cudaSuccess ||
+        (e = workspace_alloc((void**)&k0, maxE * 4, st)) != cudaSuccess ||
+        (e = workspace_alloc((void**)&k1, maxE * 4, st)) != cudaSuccess ||
+        (e = workspace_alloc((void**)&v0, maxE * 4, st)) != cudaSuccess ||
+        (e = workspace_alloc((void**)&v1, maxE * 4, st)) != cudaSuccess ||
+        (e = workspace_alloc((void**)&ctr, 8 * 4, st)) != cudaSuccess) {
         cleanup();
         return e;
     }
+    err = reinterpret_cast<int*>(ctr + 1);
     // Sort on the low key_bits bits: every valid key is < n < 2^key_bits and
     // the "no edge" key 0xffffffff reads as 2^key_bits - 1, so it sorts last.
     int key_bits = 1;
     while (key_bits < 32 && ((int64_t)1 << key_bits) <= n) ++key_bits;
     e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k0, k1, v0, v1, (int)maxE, 0, key_bits, st);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes);
+    if (e == cudaSuccess) e = workspace_alloc(&tmp, tmp_bytes, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, 4, st);
-    if (e == cudaSuccess && kind == SONG_KIND_L2 && byte_rows(range, dim)) {
+    BaseRange range;
+    if (e == cudaSuccess && kind == SONG_KIND_L2 && dim <= kU8MaxDim)
+        e = scan_base_range(static_cast<const float*>(d_base), n, dim, ld, err + 1, st, &range);
+    if (e == cudaSuccess && byte_rows(range, dim)) {
         u8_ld = u8_row_bytes(dim);
-        e = device_alloc((void**)&u8, (size_t)n * u8_ld);
+        e = workspace_alloc((void**)&u8, (size_t)n * u8_ld, st);
         if (e == cudaSuccess)
             e = convert_rows_u8(static_cast<const float*>(d_base), n, dim, ld, u8, u8_ld, st);
     }
@@ -213,8 +220,8 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
         e = cudaGetLastError();
         s += B;
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cleanup();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e;
 }
 

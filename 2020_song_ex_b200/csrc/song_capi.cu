@@ -87,10 +87,12 @@ struct song_index {
         float* edist = nullptr;
         void* split = nullptr;
         size_t split_bytes = 0;
+        int* counters = nullptr;  // arrival counters, zero between launches
         int cap_nq = 0;
     };
     static constexpr int kEntryRing = 16;
     EntrySlot eslot[kEntryRing];
+    char* eslot_mem = nullptr;  // the slots' buffers, one allocation
     unsigned eslot_next = 0;
     // learned entry / stop models
     bool has_model = false;
@@ -179,11 +181,7 @@ void free_index(song_index* x) {
     cudaFree(x->d_entry_tiles);
     cudaFree(x->d_entry_norm);
     if (x->pool) cudaMemPoolDestroy(x->pool);  // released once its async frees complete
-    for (auto& sl : x->eslot) {
-        cudaFree(sl.ecand);
-        cudaFree(sl.edist);
-        cudaFree(sl.split);
-    }
+    cudaFree(x->eslot_mem);
     cudaFree(x->d_bf16);
     cudaFree(x->d_fp8);
     cudaFree(x->d_fp8_scale);
@@ -221,7 +219,6 @@ song_status create_common(int kind, const void* rows, int64_t n, int dim, const 
     x->dim = dim;
     x->ld = song::search_row_stride(kind, dim);
     x->p = *params;
-    if (kind == SONG_KIND_L2) x->range = song::scan_base_range((const float*)rows, n, dim);
     cudaError_t e = cudaGetDevice(&x->device);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&x->num_sms, cudaDevAttrMultiProcessorCount, x->device);
@@ -260,7 +257,9 @@ song_status create_common(int kind, const void* rows, int64_t n, int dim, const 
     // a pageable cudaMemcpy may return before its DMA lands: finish the legacy
     // stream before x->stream (non-blocking) reads the uploaded rows and adjacency
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-    if (e == cudaSuccess && kind == SONG_KIND_L2 && song::byte_rows(x->range, dim)) {
+    if (e == cudaSuccess && kind == SONG_KIND_L2 && dim <= song::kU8MaxDim)
+        e = song::scan_base_range((const float*)x->d_base, n, dim, x->ld, x->d_err + 8, x->stream, &x->range);
+    if (e == cudaSuccess && song::byte_rows(x->range, dim)) {
         x->u8_ld = song::u8_row_bytes(dim);
         e = song::device_alloc((void**)&x->d_u8, (size_t)n * x->u8_ld);
         if (e == cudaSuccess)
@@ -474,25 +473,32 @@ song_status entry_slot(song_index* x, int nq, song_index::EntrySlot** out) {
         SONG_CUDA(cudaDeviceSynchronize(), "entry ring growth");
         int cap = std::max(nq, 1024);
         for (auto& r : x->eslot) cap = std::max(cap, r.cap_nq);
-        const size_t cells = (size_t)cap * song::kEntryK;
-        const size_t sb = song::entry_split_scratch_bytes(cap, x->num_sms);
-        for (auto& r : x->eslot) {
-            cudaFree(r.ecand);
-            cudaFree(r.edist);
-            cudaFree(r.split);
-            r = song_index::EntrySlot();
-            cudaError_t e = cudaMalloc(&r.ecand, cells * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&r.edist, cells * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&r.split, sb);
-            if (e == cudaSuccess) e = cudaMemset(r.split, 0, sb);  // arrival counters start at zero
-            if (e != cudaSuccess) {
-                cudaFree(r.ecand);
-                cudaFree(r.edist);
-                cudaFree(r.split);
-                r = song_index::EntrySlot();
-                return cuda_fail(e, "entry ring slot");
-            }
+        // one allocation for all slots (48 separate ones made a learned index's
+        // first search take tens of ms); only the arrival counters must start at zero
+        auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+        const size_t cells = up((size_t)cap * song::kEntryK * 4);
+        const size_t sb = up(song::entry_split_scratch_bytes(cap, x->num_sms));
+        const size_t cb = up(song::entry_split_counter_bytes(cap));
+        const size_t pitch = cb + sb + 2 * cells;
+        for (auto& r : x->eslot) r = song_index::EntrySlot();
+        cudaFree(x->eslot_mem);
+        x->eslot_mem = nullptr;
+        cudaError_t e = song::device_alloc((void**)&x->eslot_mem, pitch * song_index::kEntryRing);
+        if (e == cudaSuccess)
+            e = cudaMemset2D(x->eslot_mem, pitch, 0, cb, song_index::kEntryRing);
+        if (e != cudaSuccess) {
+            cudaFree(x->eslot_mem);
+            x->eslot_mem = nullptr;
+            return cuda_fail(e, "entry ring slot");
+        }
+        for (int i = 0; i < song_index::kEntryRing; ++i) {
+            song_index::EntrySlot& r = x->eslot[i];
+            char* m = x->eslot_mem + (size_t)i * pitch;
+            r.counters = reinterpret_cast<int*>(m);
+            r.split = m + cb;
             r.split_bytes = sb;
+            r.ecand = reinterpret_cast<int32_t*>(m + cb + sb);
+            r.edist = reinterpret_cast<float*>(m + cb + sb + cells);
             r.cap_nq = cap;
         }
     }
@@ -514,7 +520,8 @@ song_status launch(song_index* x, song::SearchArgs a, cudaStream_t st) {
         cudaError_t e = song::launch_entry((const float*)a.queries, x->dim, a.nq, x->dim,
                                            x->d_entry_tiles, x->d_entry_norm, x->d_entry_ids,
                                            x->entry_hpad, sl->ecand, sl->edist, x->d_err, st,
-                                           sl->split, sl->split_bytes, x->num_sms, true, keep);
+                                           sl->split, sl->split_bytes, x->num_sms, true, keep,
+                                           sl->counters);
         if (e != cudaSuccess) return cuda_fail(e, "entry launch");
         a.ecand = sl->ecand;
         a.edist = sl->edist;
@@ -661,26 +668,6 @@ bool byte_rows(const BaseRange& r, int dim) {
     return r.int_base && r.lo >= 0.0f && r.hi <= 255.0f && dim <= kU8MaxDim;
 }
 
-BaseRange scan_base_range(const float* rows, int64_t n, int dim) {
-    BaseRange r;
-    const int64_t total = n * (int64_t)dim;
-    if (total <= 0) return r;
-    float lo = rows[0], hi = rows[0];
-    bool integral = true;
-    for (int64_t i = 0; i < total; ++i) {
-        const float v = rows[i];
-        if (!(v == std::nearbyint(v)) || !(std::fabs(v) < 16777216.0f)) {
-            integral = false;
-            break;
-        }
-        lo = v < lo ? v : lo;
-        hi = v > hi ? v : hi;
-    }
-    r.int_base = integral ? 1 : 0;
-    r.lo = lo;
-    r.hi = hi;
-    return r;
-}
 }  // namespace song
 
 extern "C" {
@@ -779,8 +766,6 @@ song_status song_build_graph(int kind, const void* rows, int64_t n, int dim,
     const int ratio = batch_ratio > 0 ? batch_ratio : 32;
     const int bfw = build_bf_words > 0 ? build_bf_words : 1024;
     const int ld = song::search_row_stride(kind, dim);
-    const song::BaseRange range =
-        kind == SONG_KIND_L2 ? song::scan_base_range((const float*)rows, n, dim) : song::BaseRange();
     int dev = 0, sms = 0;
     SONG_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
     SONG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
@@ -788,24 +773,26 @@ song_status song_build_graph(int kind, const void* rows, int64_t n, int dim,
     int32_t* d_adj = nullptr;
     cudaStream_t st = nullptr;
     const size_t row_bytes = (size_t)ld * 4;
-    cudaError_t e = song::device_alloc(&d_rows, (size_t)n * row_bytes);
-    if (e == cudaSuccess) e = song::device_alloc((void**)&d_adj, (size_t)n * params->block_size * 4);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess && ld != dim) e = cudaMemset(d_rows, 0, (size_t)n * row_bytes);
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = song::workspace_alloc(&d_rows, (size_t)n * row_bytes, st);
     if (e == cudaSuccess)
-        e = cudaMemcpy2D(d_rows, row_bytes, rows, (size_t)dim * 4, (size_t)dim * 4, (size_t)n,
-                         cudaMemcpyHostToDevice);
-    // a pageable copy may return before its DMA lands, and st does not wait for
-    // the legacy stream
-    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        e = song::workspace_alloc((void**)&d_adj, (size_t)n * params->block_size * 4, st);
+    if (e == cudaSuccess && ld != dim) e = cudaMemsetAsync(d_rows, 0, (size_t)n * row_bytes, st);
     if (e == cudaSuccess)
-        e = song::build_graph_device(kind, d_rows, n, dim, ld, *params, ratio, bfw, d_adj,
-                                     sms, st, range);
+        e = cudaMemcpy2DAsync(d_rows, row_bytes, rows, (size_t)dim * 4, (size_t)dim * 4, (size_t)n,
+                              cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
-        e = cudaMemcpy(adj_out, d_adj, (size_t)n * params->block_size * 4, cudaMemcpyDeviceToHost);
-    cudaFree(d_rows);
-    cudaFree(d_adj);
-    if (st) cudaStreamDestroy(st);
+        e = song::build_graph_device(kind, d_rows, n, dim, ld, *params, ratio, bfw, d_adj, sms, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(adj_out, d_adj, (size_t)n * params->block_size * 4,
+                            cudaMemcpyDeviceToHost, st);
+    if (st) {
+        if (d_rows) cudaFreeAsync(d_rows, st);
+        if (d_adj) cudaFreeAsync(d_adj, st);
+        const cudaError_t es = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = es;
+        cudaStreamDestroy(st);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "graph build");
     return SONG_OK;
 }

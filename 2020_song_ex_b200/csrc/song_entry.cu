@@ -497,6 +497,8 @@ static size_t tile_done_bytes(int nq) {
     return (qt * 4 + 255) / 256 * 256;
 }
 
+size_t entry_split_counter_bytes(int nq) { return tile_done_bytes(nq); }
+
 size_t entry_split_scratch_bytes(int nq, int num_sms) {
     const int qt = (nq + kM - 1) / kM;
     int splits = qt <= 1 ? kEntrySplits : (2 * num_sms) / qt;
@@ -508,7 +510,7 @@ cudaError_t launch_entry(const float* d_queries, int qld, int nq, int dim,
                          const __nv_bfloat16* d_tiles, const float* d_norm, const int32_t* d_ids,
                          int hpad, int32_t* d_out_ids, float* d_out_d, int* d_err,
                          cudaStream_t st, void* split_scratch, size_t split_bytes, int num_sms,
-                         bool overlap, int keep) {
+                         bool overlap, int keep, int* counters) {
     if (nq <= 0) return cudaSuccess;
     if (dim > kEntryMaxDim || hpad % kN != 0 || hpad <= 0) return cudaErrorInvalidValue;
     EntryArgs a;
@@ -531,13 +533,13 @@ cudaError_t launch_entry(const float* d_queries, int qld, int nq, int dim,
     const int qt = (nq + kM - 1) / kM;
     int splits = qt <= 1 ? kEntrySplits : (2 * num_sms) / qt;
     splits = std::max(1, std::min(std::min(kEntrySplits, a.ntiles), splits));
-    const size_t per_split = (size_t)nq * kK * 8, head = tile_done_bytes(nq);
+    const size_t per_split = (size_t)nq * kK * 8, head = counters != nullptr ? 0 : tile_done_bytes(nq);
     if (split_scratch == nullptr || split_bytes < head) splits = 1;
     else splits = (int)std::min<size_t>((size_t)splits, (split_bytes - head) / per_split);
     if (splits < 1) splits = 1;
     a.tiles_per_split = (a.ntiles + splits - 1) / splits;
     splits = (a.ntiles + a.tiles_per_split - 1) / a.tiles_per_split;
-    a.tile_done = static_cast<int*>(split_scratch);
+    a.tile_done = counters != nullptr ? counters : static_cast<int*>(split_scratch);
     a.part_key = reinterpret_cast<float*>(static_cast<char*>(split_scratch) + head);
     a.part_idx = reinterpret_cast<int32_t*>(static_cast<char*>(split_scratch) + head +
                                             (size_t)splits * nq * kK * 4);

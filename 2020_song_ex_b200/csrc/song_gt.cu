@@ -808,6 +808,15 @@ void trim_workspaces(int dev) {
     if (g_pool[dev] != nullptr) cudaMemPoolTrimTo(g_pool[dev], 0);
 }
 
+cudaError_t workspace_alloc(void** p, size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = workspace_pool(dev, &pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    return e;
+}
+
 cudaError_t device_alloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
@@ -848,9 +857,7 @@ cudaError_t exact_knn(const float* d_base, int64_t n, int64_t ldb, int dim, cons
     const size_t o_flags = take(3 * sizeof(int));  // [0] query lo, [1] base lo, [2] error word
     const size_t o_bound = take((size_t)nq * 4);
     char* ws = nullptr;
-    cudaMemPool_t pool = nullptr;
-    e = workspace_pool(dev, &pool);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), total, pool, st);
+    e = workspace_alloc(reinterpret_cast<void**>(&ws), total, st);
     if (e != cudaSuccess) return e;
     int* flags = reinterpret_cast<int*>(ws + o_flags);
     e = cudaMemsetAsync(flags, 0, 3 * sizeof(int), st);

@@ -98,6 +98,7 @@ cudaError_t build_entry_tables(const float* d_base, int ld, int dim, const int32
 // asynchronous memset on the stream before each launch).
 constexpr int kEntrySplits = 16;
 size_t entry_split_scratch_bytes(int nq, int num_sms);
+size_t entry_split_counter_bytes(int nq);  // the arrival counters in front of it
 // overlap: the scratch's arrival counters are zero (the kernel leaves them
 // so) and the launch may start while the previous search launch on the stream
 // finishes its tail; it ends after that launch.  Otherwise a memset zeroes the
@@ -105,11 +106,15 @@ size_t entry_split_scratch_bytes(int nq, int num_sms);
 // keep: how many of the nearest hubs the caller reads (the rest of each
 // kEntryK row is -1 / +inf); the first `keep` entries are those of the full
 // list.  kEntryK for the entry model's features.
+// counters: the arrival counters apart from the scratch (entry_split_counter_bytes
+// of the largest nq, zero), for a scratch that calls of several nq take in turn:
+// in front of it their place would depend on nq and the lists of a small call
+// would overwrite the counters of a larger one.
 cudaError_t launch_entry(const float* d_queries, int qld, int nq, int dim,
                          const __nv_bfloat16* d_tiles, const float* d_norm, const int32_t* d_ids,
                          int hpad, int32_t* d_out_ids, float* d_out_d, int* d_err,
                          cudaStream_t st, void* split_scratch, size_t split_bytes, int num_sms,
-                         bool overlap = false, int keep = kEntryK);
+                         bool overlap = false, int keep = kEntryK, int* counters = nullptr);
 
 // Graph::search (graph.h:33-115) bit for bit (song_graphsearch.cu).
 int graph_search_frontier_cap(int ef);
@@ -130,14 +135,17 @@ int lowp_padded_dim(int prec, int dim);
 cudaError_t quantize_rows(int prec, const float* d_rows, int64_t n, int dim, int ld, void* d_out,
                           int out_ld, float* d_scales, cudaStream_t st);
 
-// Integer range of FP32 rows (0 in int_base if any value is not an integer).
+// Integer range of FP32 rows (int_base 0 if any value is not an integer).
 struct BaseRange {
     int int_base = 0;
     float lo = 0.0f, hi = 0.0f;
 };
+// Scans device rows [n x ld]; d_scratch: 3 ints.  Synchronises st.  (On one
+// host thread the scan took a third of the time of a 100,000 x 128 build.)
+cudaError_t scan_base_range(const float* d_rows, int64_t n, int dim, int ld, int* d_scratch,
+                            cudaStream_t st, BaseRange* out);
 // Rows that may be kept as bytes (convert_rows_u8).
 bool byte_rows(const BaseRange& r, int dim);
-BaseRange scan_base_range(const float* rows, int64_t n, int dim);
 
 // Byte rows of integer-valued vectors: at most kU8MaxDim elements, each row
 // zero padded to u8_row_bytes(dim) (a multiple of 16) -- the exact-integer
@@ -160,7 +168,7 @@ cudaError_t launch_search(int kind, const SearchArgs& a, int num_sms, cudaStream
 // Batched-insertion NSW build over device rows (song_build.cu).
 cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim, int ld,
                                const song_params& p, int ratio, int bf_words, int32_t* d_adj,
-                               int num_sms, cudaStream_t st, BaseRange range = BaseRange());
+                               int num_sms, cudaStream_t st);
 
 // Scratch bytes build_graph_with_scratch needs for (n, params, ratio).
 size_t build_scratch_bytes(int64_t n, const song_params& p, int ratio);
@@ -241,6 +249,8 @@ cudaError_t index_entry(song_index* x, const float* d_q, int qld, int nq, int32_
 // back; cudaMalloc that does so before it fails.
 void trim_workspaces(int dev);
 cudaError_t device_alloc(void** p, size_t bytes);
+// A block of that pool, stream-ordered on st; freed with cudaFreeAsync on st.
+cudaError_t workspace_alloc(void** p, size_t bytes, cudaStream_t st);
 
 // Records a failure message for song_last_error() on the calling thread.
 song_status set_error(song_status status, const char* message);

@@ -2,6 +2,8 @@
 // song_search.cuh, their instances in song_search_*.cu).
 #include "song_search.cuh"
 
+#include <cstring>
+
 namespace song {
 
 std::atomic<int64_t> g_launches{0};
@@ -15,6 +17,41 @@ __global__ void rows_to_u8(const float* __restrict__ x, int64_t n, int dim, int 
     if (r >= n) return;
     for (int i = threadIdx.x; i < out_ld; i += blockDim.x)
         out[r * out_ld + i] = i < dim ? (uint8_t)x[r * ld + i] : (uint8_t)0;
+}
+
+// Order-preserving map of a float to an int, for atomicMin / atomicMax.
+__device__ __forceinline__ int ord_int(float x) {
+    const int b = __float_as_int(x);
+    return b >= 0 ? b : b ^ 0x7fffffff;
+}
+
+// out[0] := 1 if some value is not an integer of magnitude below 2^24, out[1]
+// and out[2] the smallest and largest value in ord_int order (of the values
+// before the first block saw such a one).  One pass over the rows.
+__global__ void scan_rows(const float* __restrict__ x, int64_t n, int dim, int ld, int* __restrict__ out) {
+    float lo = INFINITY, hi = -INFINITY;
+    bool bad = false;
+    const int64_t total = n * (int64_t)dim, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
+        const float v = __ldg(x + (ld == dim ? i : (i / dim) * ld + i % dim));
+        bad |= !(v == rintf(v)) || !(fabsf(v) < 16777216.0f);
+        lo = fminf(lo, v);
+        hi = fmaxf(hi, v);
+    }
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(FULL, lo, w));
+        hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, w));
+    }
+    bad = __any_sync(FULL, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (bad) {
+            out[0] = 1;
+        } else {
+            atomicMin(out + 1, ord_int(lo));
+            atomicMax(out + 2, ord_int(hi));
+        }
+    }
 }
 
 // FP32 -> BF16 (round to nearest even) rows, zero padded to out_ld bytes.
@@ -138,6 +175,31 @@ cudaError_t convert_rows_u8(const float* d_rows, int64_t n, int dim, int ld, uin
     if (n <= 0) return cudaSuccess;
     rows_to_u8<<<(unsigned)n, 128, 0, st>>>(d_rows, n, dim, ld, d_out, out_ld);
     return cudaGetLastError();
+}
+
+cudaError_t scan_base_range(const float* d_rows, int64_t n, int dim, int ld, int* d_scratch,
+                            cudaStream_t st, BaseRange* r) {
+    *r = BaseRange();
+    if (n <= 0 || dim <= 0) return cudaSuccess;
+    int h[3] = {0, INT_MAX, INT_MIN};
+    cudaError_t e = cudaMemcpyAsync(d_scratch, h, sizeof h, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return e;
+    const int64_t blocks = std::min<int64_t>((n * (int64_t)dim + 255) / 256, 148 * 8);
+    scan_rows<<<(unsigned)blocks, 256, 0, st>>>(d_rows, n, dim, ld, d_scratch);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_scratch, sizeof h, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess || h[0] != 0) return e;
+    auto value = [](int o) {
+        const int b = o >= 0 ? o : o ^ 0x7fffffff;
+        float f;
+        std::memcpy(&f, &b, sizeof f);
+        return f;
+    };
+    r->int_base = 1;
+    r->lo = value(h[1]);
+    r->hi = value(h[2]);
+    return cudaSuccess;
 }
 
 int search_row_stride(int kind, int dim) {
