@@ -277,7 +277,24 @@ __device__ __forceinline__ unsigned long long kth_bound(const unsigned long long
         }
     unsigned long long lo = (unsigned long long)__reduce_min_sync(0xffffffffu, mn) << 32;
     unsigned long long hi = ((unsigned long long)__reduce_max_sync(0xffffffffu, mx) << 32) | 0xfffffffeu;
-    while (lo < hi) {  // at most 64 rounds
+    while (E > 2 && hi - lo > 3) {  // four parts per round: the three counts (at most 256) in one redux
+        const unsigned long long step = (hi - lo) >> 2;
+        const unsigned long long p1 = lo + step, p2 = p1 + step, p3 = p2 + step;
+        unsigned c = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            c += (key[e] <= p1 ? 1u : 0u) + (key[e] <= p2 ? 1u << 10 : 0u) + (key[e] <= p3 ? 1u << 20 : 0u);
+        c = __reduce_add_sync(0xffffffffu, c);
+        const unsigned c1 = c & 1023u, c2 = (c >> 10) & 1023u, c3 = c >> 20, want = (unsigned)k;
+        if (c1 == want) return p1;
+        if (c2 == want) return p2;
+        if (c3 == want) return p3;
+        if (c1 > want) hi = p1;
+        else if (c2 > want) { lo = p1 + 1; hi = p2; }
+        else if (c3 > want) { lo = p2 + 1; hi = p3; }
+        else lo = p3 + 1;
+    }
+    while (lo < hi) {
         const unsigned long long mid = lo + ((hi - lo) >> 1);
         unsigned c = 0;
 #pragma unroll
@@ -583,13 +600,27 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
                     m1 = fminf(fminf(m1, v[4 * g + 2]), v[4 * g + 3]);
                 }
                 if (!__any_sync(FULL, !(fminf(m0, m1) >= thr))) return;
-                // the columns some lane of the warp may take, one at a time: few, and the
-                // code stays small (32 unrolled copies of the exact test overflowed the
-                // instruction cache: 7,000 cycles per chunk with one key below the threshold)
+                // the columns some lane of the warp may take: few of them one at a time (32
+                // unrolled copies with a branch each took 7,000 cycles per chunk with one key
+                // below the threshold), many of them all, without branches (one at a time is
+                // 150 cycles per column: while the lists of a large k first fill, 4,800)
                 unsigned mine = 0u;
 #pragma unroll
                 for (int jj = 0; jj < 32; ++jj) mine |= (v[jj] >= thr ? 0u : 1u) << jj;
                 unsigned todo = __reduce_or_sync(FULL, mine);
+                if (CAP > 64 && __popc(todo) > 8) {
+                    const int64_t left = a.n - (col0 + c0);
+#pragma unroll
+                    for (int jj = 0; jj < 32; ++jj) {
+                        const float cross2 = 2.0f * __uint_as_float(r[jj]);
+                        const float d = __fadd_rn(__fadd_rn(__fsub_rn(qn, cross2), bn[c0 + jj]), 0.0f);
+                        const uint32_t o = ord32(d);
+                        const bool in = ((mine >> jj) & 1u) && o < lim && jj < left;
+                        if (in) list[cnt] = ((unsigned long long)o << 32) | (uint32_t)(col0 + c0 + jj);
+                        cnt += in;
+                    }
+                    todo = 0u;
+                }
                 while (todo) {
                     const int jj = __ffs(todo) - 1;
                     todo &= todo - 1u;
@@ -607,6 +638,7 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
                     }
                     __syncwarp();
                 }
+                __syncwarp();
                 unsigned full = __ballot_sync(FULL, cnt > CAP - 32);
                 while (full) {  // cut the list of lane s to its k smallest keys
                     const int s = __ffs(full) - 1;
