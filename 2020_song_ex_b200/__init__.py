@@ -459,9 +459,9 @@ def gpu_search(g, queries, nq: int, k: int, N_MULTIQUERY: int = 512, ef_search: 
         fn = L.song_gpu_search_hamming
     ids = np.empty(max(nq * k, 1), dtype=np.int32)
     tq = np.zeros((nq, 12), dtype=np.int32) if trace is not None else None
-    t = _Timing()
+    t = _Timing()  # times cost four events per batch: only for a trace
     _check(fn(g._h, q.ctypes.data, nq, k, N_MULTIQUERY, ef, ids.ctypes.data,
-              tq.ctypes.data if tq is not None else None, C.byref(t)))
+              tq.ctypes.data if tq is not None else None, C.byref(t) if trace is not None else None))
     if trace is not None:
         trace.ef_search, trace.batch_limit = t.ef_search, t.batch_limit
         trace.alloc_ms, trace.h2d_ms, trace.memset_ms = t.alloc_ms, t.h2d_ms, t.memset_ms
