@@ -40,12 +40,13 @@
 // this split in global memory (fire and forget); a list that fills up is cut
 // by its warp to its k smallest keys, the k-th becoming the threshold.  A
 // query's splits share their smallest threshold through one word per query
-// in global memory: any split's k-th distance bounds the final one.  A
+// in global memory: any split's k-th distance bounds the final one (and, with
+// many splits, their ceil(k / splits)-th distances together: kMaxUm).  A
 // max-heap per query in shared memory instead made every insertion a chain
 // of dependent shared accesses, one query tile of 4 warps per SM and a
 // separate threshold per split.  Whole calls: 10,000 queries x 1M x 128
 // integers at k = 10 17.6 -> 3.7 ms (the kernel 17.3 -> 3.5 ms, 0.73 PFLOP/s),
-// at k = 100 36.7 -> 7.3 ms; 777 x 99,991 x 100 floats at k = 100 2.2 -> 0.56
+// at k = 100 36.7 -> 7.3 ms; 777 x 99,991 x 100 floats at k = 100 2.2 -> 0.44
 // ms; 50 x 5,000 x 24 at k = 1 0.71 -> 0.10 ms.
 //
 // A key that ties a split's own threshold has a larger id than the k kept
@@ -261,8 +262,21 @@ struct GtArgs {
     unsigned long long* list;     // [nq][splits][CAP] keys, unordered
     int* count;                   // [nq][splits]
     uint32_t* bound;              // [nq] ordered bits of the smallest k-th distance of any split
+    uint32_t* nth;                // [splits][nq] ordered bits of a split's um-th smallest distance
+    int um, used;                 // ceil(k / used), or 0: not used; the splits that have a tile
     int* err;                     // set to 2 when a bounded wait gives up
 };
+
+// While lists of a large k fill, the splits of a query also share their um-th
+// smallest distances, um = ceil(k / splits): the largest of these bounds the
+// final k-th too (um of every split lie at or below it, k together), and it is
+// there after the first tile, where a split's own k-th distance takes a full
+// list and its cut.  A split keeps its um smallest in registers, so only for um
+// <= 4: few queries, many splits (777 x 99,991 x 100 at k = 100, 36 splits,
+// 0.57 -> 0.44 ms; 100 x 500,000 x 128 at k = 100 0.61 -> 0.48; 1,500 x 60,000 x
+// 200 at k = 32 0.45 -> 0.41).  In instances of their own: compiled into the
+// others and switched off it cost 10,000 x 1M at k = 100 23 %.
+constexpr int kMaxUm = 4;
 
 // A value t with exactly k of the valid keys (not ~0) <= t: bisection of the
 // key range (keys are unique and at least k are valid).  E keys per lane.
@@ -351,7 +365,7 @@ __device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
 
 // MT: query tiles per CTA.  CAP: list entries per query and split (a
 // multiple of 32, at least k + 32, so that a chunk always fits).
-template <int MT, int CAP>
+template <int MT, int CAP, bool UM>
 __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a) {
     constexpr int EW = 4 * MT;  // epilogue warps
     constexpr unsigned FULL = 0xffffffffu;
@@ -571,11 +585,34 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
         set_limit(live ? *(volatile const uint32_t*)(a.bound + q) : 0u);
         const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * kN);
         uint32_t seen = 0xFFFFFFFFu;  // the shared bound, read one tile before it is used
+        uint32_t low[kMaxUm];         // this split's smallest distances, ascending
+#pragma unroll
+        for (int i = 0; i < kMaxUm; ++i) low[i] = 0xFFFFFFFFu;
+        auto lowest = [&](uint32_t o) {
+#pragma unroll
+            for (int i = 0; i < kMaxUm; ++i) {
+                const uint32_t m = min(low[i], o);
+                o = max(low[i], o);
+                low[i] = m;
+            }
+        };
+        uint32_t said = 0xFFFFFFFFu;  // the last one written to a.nth
         for (int j = 0; j < ntl; ++j) {
             const int b = j & 1;
             const float* bn = bn_s[j % kNormSlots];
             if (live && (j & 3) == 3) set_limit(seen);
             if (live && (j & 3) == 2) seen = *(volatile const uint32_t*)(a.bound + q);
+            if (UM && live && (j < 8 || (j & 3) == 3)) {
+                const uint32_t mine = a.um == 1 ? low[0] : a.um == 2 ? low[1] : a.um == 3 ? low[2] : low[3];
+                if (mine < said) *(volatile uint32_t*)(a.nth + (size_t)y * a.nq + q) = said = mine;
+                uint32_t t = 0u;
+#pragma unroll 8
+                for (int i = 0; i < a.used; ++i) t = max(t, *(volatile const uint32_t*)(a.nth + (size_t)i * a.nq + q));
+                if (t < seen) {
+                    seen = min(atomicMin(a.bound + q, t), t);
+                    set_limit(seen);
+                }
+            }
             bool ok = mbar_wait(smem_addr(&bar_accf[b]), (uint32_t)((j >> 1) & 1), &abort_flag);
             ok = __all_sync(FULL, ok);
             if (!ok) {
@@ -618,6 +655,7 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
                         const bool in = ((mine >> jj) & 1u) && o < lim && jj < left;
                         if (in) list[cnt] = ((unsigned long long)o << 32) | (uint32_t)(col0 + c0 + jj);
                         cnt += in;
+                        if constexpr (UM) lowest(in ? o : 0xFFFFFFFFu);
                     }
                     todo = 0u;
                 }
@@ -633,8 +671,10 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
                         const float cross2 = 2.0f * __uint_as_float(x);
                         const float d = __fadd_rn(__fadd_rn(__fsub_rn(qn, cross2), bn[c0 + jj]), 0.0f);
                         const uint32_t o = ord32(d);
-                        if (o < lim && col0 + c0 + jj < a.n)
+                        if (o < lim && col0 + c0 + jj < a.n) {
                             list[cnt++] = ((unsigned long long)o << 32) | (uint32_t)(col0 + c0 + jj);
+                            if constexpr (UM) lowest(o);
+                        }
                     }
                     __syncwarp();
                 }
@@ -888,12 +928,17 @@ cudaError_t exact_knn(const float* d_base, int64_t n, int64_t ldb, int dim, cons
     const size_t o_list = take((size_t)nq * splits * cap * 8), o_cnt = take((size_t)nq * splits * 4);
     const size_t o_flags = take(3 * sizeof(int));  // [0] query lo, [1] base lo, [2] error word
     const size_t o_bound = take((size_t)nq * 4);
+    const int tps = (ntiles + splits - 1) / splits, used = (ntiles + tps - 1) / tps;
+    int um = (k + used - 1) / used;
+    if (cap == 64 || used == 1 || um > kMaxUm) um = 0;
+    const size_t o_nth = take(um ? (size_t)nq * splits * 4 : 0);
     char* ws = nullptr;
     e = workspace_alloc(reinterpret_cast<void**>(&ws), total, st);
     if (e != cudaSuccess) return e;
     int* flags = reinterpret_cast<int*>(ws + o_flags);
     e = cudaMemsetAsync(flags, 0, 3 * sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws + o_bound, 0xff, (size_t)nq * 4, st);
+    if (e == cudaSuccess && um) e = cudaMemsetAsync(ws + o_nth, 0xff, (size_t)nq * splits * 4, st);
     int h_err = 0;
     if (e == cudaSuccess) {
         const auto vec = [](const float* p, int64_t ld) {
@@ -916,15 +961,21 @@ cudaError_t exact_knn(const float* d_base, int64_t n, int64_t ldb, int dim, cons
         a.n = (int)n;
         a.nch = nch;
         a.ntiles = ntiles;
-        a.tiles_per_split = (ntiles + splits - 1) / splits;
+        a.tiles_per_split = tps;
         a.splits = splits;
         a.k = k;
         a.list = reinterpret_cast<unsigned long long*>(ws + o_list);
         a.count = reinterpret_cast<int*>(ws + o_cnt);
         a.bound = reinterpret_cast<uint32_t*>(ws + o_bound);
+        a.nth = reinterpret_cast<uint32_t*>(ws + o_nth);
+        a.um = um;
+        a.used = used;
         a.err = flags + 2;
-        void (*kern)(const GtArgs) = mt == 2 ? (cap == 64 ? gt_kernel<2, 64> : gt_kernel<2, 256>)
-                                             : (cap == 64 ? gt_kernel<1, 64> : gt_kernel<1, 256>);
+        void (*kern)(const GtArgs) = mt == 2 ? gt_kernel<2, 64, false> : gt_kernel<1, 64, false>;
+        if (cap == 256) {
+            kern = mt == 2 ? gt_kernel<2, 256, false> : gt_kernel<1, 256, false>;
+            if (um) kern = mt == 2 ? gt_kernel<2, 256, true> : gt_kernel<1, 256, true>;
+        }
         cudaFuncAttributes fa;
         e = cudaFuncGetAttributes(&fa, kern);
         if (e == cudaSuccess) {

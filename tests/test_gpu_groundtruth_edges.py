@@ -68,3 +68,20 @@ def test_calls_on_two_threads(cuda):
         for ids, d in out[i]:
             np.testing.assert_array_equal(ids, ref_ids)
             np.testing.assert_array_equal(d, ref_d.astype(np.float32))
+
+
+@pytest.mark.parametrize("n,nq,k", [(20000, 130, 17), (20000, 130, 100), (40000, 7, 128), (9000, 257, 64)])
+@pytest.mark.parametrize("order", ["ascending", "descending"])
+def test_neighbours_in_one_split(cuda, n, nq, k, order):
+    """Bases sorted by their distance from where the queries lie: all neighbours
+    come from the first split, or from the last one."""
+    rng = np.random.default_rng(n + k)
+    level = np.sort(rng.integers(0, 200, size=n))
+    base = (level[:, None] + rng.integers(0, 8, size=(n, 24))).astype(np.float32)
+    if order == "descending":
+        base = base[::-1].copy()
+    q = rng.integers(0, 8, size=(nq, 24)).astype(np.float32)
+    ids, d = _gt().knn(base, q, k)
+    ref_ids, ref_d = _exact_int(base, q, k)
+    np.testing.assert_array_equal(ids, ref_ids)
+    np.testing.assert_array_equal(d, ref_d.astype(np.float32))
