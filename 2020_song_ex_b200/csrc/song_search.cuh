@@ -777,14 +777,19 @@ __device__ __forceinline__ unsigned bloom_new(const BloomRow& br, unsigned fresh
 
 // Four floats of the query from element i on: 16 aligned bytes of shared
 // memory (QG = 0, zero padded to a multiple of 4), or the caller's own row in
-// global memory (QG = 1, any alignment, zero past dim).
+// global memory (any alignment, zero past dim): QG = 1 through the read-only
+// path, QG = 2 with plain loads, for the serving kernel, whose request slots
+// are rewritten while it runs.  (For QG = 1 too, plain loads took 8 % longer at
+// 200 dimensions and queue 200, through their registers, and loads from L2 up
+// to 37 %.)
 template <int QG>
 __device__ __forceinline__ float4 query4(const float* q, int i, int dim) {
-    if constexpr (QG) {
-        return make_float4(__ldg(q + i), i + 1 < dim ? __ldg(q + i + 1) : 0.0f,
-                           i + 2 < dim ? __ldg(q + i + 2) : 0.0f, i + 3 < dim ? __ldg(q + i + 3) : 0.0f);
-    } else {
+    if constexpr (QG == 0) {
         return *reinterpret_cast<const float4*>(q + i);
+    } else {
+        auto at = [&](int j) { return QG == 1 ? __ldg(q + j) : *(q + j); };
+        return make_float4(at(i), i + 1 < dim ? at(i + 1) : 0.0f, i + 2 < dim ? at(i + 2) : 0.0f,
+                           i + 3 < dim ? at(i + 3) : 0.0f);
     }
 }
 
@@ -1603,8 +1608,10 @@ __device__ __forceinline__ unsigned fkey(float x) {
 // array for that queue.
 // TR = 0: the per-query trace is not written (a.trace must be null), so its
 // counters are dead code and free their registers.  TD = 1 (TM = TMC = 1):
-// the results queue's distances in TMEM too.
-template <int KIND, int NE, int GPL, int DT, int LM, int TM = 0, int TMC = TM, int TR = 1, int TD = 0, int QR = 0>
+// the results queue's distances in TMEM too.  SV = 1: called by the serving
+// kernel, whose queries lie in memory that is written while it runs.
+template <int KIND, int NE, int GPL, int DT, int LM, int TM = 0, int TMC = TM, int TR = 1, int TD = 0, int QR = 0,
+          int SV = 0>
 __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsigned char* ws,
                                              int lane, uint32_t tbase = 0) {
     static_assert(!TD || (TM && TMC), "distances in TMEM go with the ids in TMEM");
@@ -1669,6 +1676,9 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
             // byte rows hold a base in [0, 255]; a query there too makes every
             // partial sum an integer below 2^24 (dim <= 256): exact dp4a distances
             u8_mode = a.u8 != nullptr && integral && lo >= 0.0f && hi <= 255.0f;
+            // the request before this one in its slot was read through L1: no lane may be
+            // served its floats (plain loads are ordered by a fence after the claim)
+            if (SV && !u8_mode) __threadfence();
             if (u8_mode) {
                 qq = (int)__reduce_add_sync(FULL, (unsigned)s2);
 #pragma unroll
@@ -1730,7 +1740,7 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int qid, unsig
             const float* base = reinterpret_cast<const float*>(a.base);
             if constexpr (kU8) {
                 if (u8_mode) d = l2_u8<kNC, (QR > 0)>(a.u8, a.u8_ld, a.u8_ld >> 4, qb, qq, m, want, rows, lane);
-                else d = l2_rows<1>(base, a.ld, a.dim, sqg, m, want, rows, lane);
+                else d = l2_rows<1 + SV>(base, a.ld, a.dim, sqg, m, want, rows, lane);
             } else {
                 d = l2_rows<0>(base, a.ld, a.dim, sq, m, want, rows, lane);
             }
