@@ -190,7 +190,7 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
         a.dim = dim;
         a.ld = ld;
         a.qld = ld;
-        a.qdim = kind == SONG_KIND_L2 ? ld : dim;
+        a.qdim = kind == SONG_KIND_L2 ? search_row_stride(kind, dim) : dim;
         a.block_size = bs;
         a.k = sd;
         a.nq = B;
@@ -314,7 +314,8 @@ cudaError_t build_graph_with_scratch(int kind, const void* d_base, int64_t n, in
         a.dim = dim;
         a.ld = ld;
         a.qld = ld;
-        a.qdim = kind == SONG_KIND_L2 ? ld : dim;
+        // by the dimension: ld is the caller's and may be many times larger
+        a.qdim = kind == SONG_KIND_L2 ? search_row_stride(kind, dim) : dim;
         a.block_size = bs;
         a.k = sd;
         a.nq = B;

@@ -45,7 +45,8 @@ struct SearchArgs {
     const void* lowp;        // compressed rows [n x lowp_ld bytes]
     const float* scales;     // FP8: per-vector scale [n]
     int lowp_ld;             // bytes per compressed row (multiple of 128)
-    int qdim;                // floats of the query kept in shared memory (padded dim, at least ld)
+    int qdim;                // floats of the query kept in shared memory (dim padded to 4; with a
+                             // re-rank at least ld, the stride of the index's own rows)
     int rerank;              // 1: exact FP32 re-rank of the final results queue
     float* out_dist;         // [nq x k] distance of each output id (nullable)
     // learned entry / stop (lm: 0 off, 1 collect traces of the full search, 2 infer)
