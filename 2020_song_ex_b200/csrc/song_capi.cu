@@ -486,6 +486,9 @@ song_status entry_slot(song_index* x, int nq, song_index::EntrySlot** out) {
         cudaError_t e = song::device_alloc((void**)&x->eslot_mem, pitch * song_index::kEntryRing);
         if (e == cudaSuccess)
             e = cudaMemset2D(x->eslot_mem, pitch, 0, cb, song_index::kEntryRing);
+        // the memset runs on the legacy stream, which the non-blocking streams of
+        // the entry launches do not wait for
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         if (e != cudaSuccess) {
             cudaFree(x->eslot_mem);
             x->eslot_mem = nullptr;

@@ -220,6 +220,7 @@ song_status song_server_create(song_index* index, const song_server_config* cfg,
     if (e == cudaSuccess) e = cudaMalloc(&v->d_ring, (size_t)v->slots * v->slot_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&v->d_ctrl, 64);
     if (e == cudaSuccess) e = cudaMemset(v->d_ctrl, 0, 64);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // kst and cst do not wait for the legacy stream
     if (e == cudaSuccess) e = cudaHostAlloc(&v->h_stage, (size_t)v->slots * v->slot_bytes, cudaHostAllocDefault);
     if (e == cudaSuccess) e = cudaHostAlloc(&v->h_tailbuf, (size_t)v->slots * 8, cudaHostAllocDefault);
     if (e == cudaSuccess) e = cudaHostAlloc(&v->h_stop, 64, cudaHostAllocDefault);
