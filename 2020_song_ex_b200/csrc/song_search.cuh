@@ -628,6 +628,7 @@ __device__ __forceinline__ int q_push(RQueue<R>& q, unsigned N, float d, int nb,
         const int rk = (lane - q.sz) & 31;  // the push whose slot is one of this lane's
         const unsigned x = __shfl_sync(FULL, db, rk);
         if (mine && lane < a) q.id[q.sz + lane] = nb;
+        __syncwarp();
         const int key = rk < a ? (q.sz + rk) >> 5 : -1;
 #pragma unroll
         for (int r = 0; r < R; ++r) pick_if(q.d[r], r, key, x);
@@ -642,7 +643,10 @@ __device__ __forceinline__ int q_push(RQueue<R>& q, unsigned N, float d, int nb,
         while (rest) {
             const int j = __ffs(rest) - 1;
             const unsigned dj = __shfl_sync(FULL, db, j);
+            // one slot may be evicted again and again, by other lanes: redux and
+            // shuffles do not order their writes
             if (lane == j) q.id[fi] = nb;
+            __syncwarp();
             q_set_dbits(q, (int)fi, dj, lane);
             if (MIN && fi == q.nxi) q.nx = false;
             ++acc;
