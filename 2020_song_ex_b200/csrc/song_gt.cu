@@ -388,12 +388,13 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
     const uint32_t b_stage = (uint32_t)(group * b_parts) * kBlock;
     // query blocks resident when they leave room for three stages of base
     // blocks, else a stage carries both
-    const uint32_t a_bytes = (uint32_t)(MT * a_parts * a.nch) * kBlock;
-    const bool resident = a_bytes + 3u * b_stage <= a.ring_bytes;
+    const uint64_t a_bytes64 = (uint64_t)(MT * a_parts) * a.nch * kBlock;  // 2^32 at four million dimensions
+    const bool resident = a_bytes64 + 3u * b_stage <= a.ring_bytes;
+    const uint32_t a_bytes = resident ? (uint32_t)a_bytes64 : 0u;
     const uint32_t a_stage = resident ? 0u : (uint32_t)(MT * a_parts * group) * kBlock;
     const uint32_t stage_bytes = a_stage + b_stage;
-    unsigned char* ring = smem + (resident ? a_bytes : 0u);
-    const int stages = min(kMaxStages, (int)((a.ring_bytes - (resident ? a_bytes : 0u)) / stage_bytes));
+    unsigned char* ring = smem + a_bytes;
+    const int stages = min(kMaxStages, (int)((a.ring_bytes - a_bytes) / stage_bytes));
 
     const int qt = blockIdx.x, y = blockIdx.y;
     const int t_begin = y * a.tiles_per_split;
