@@ -580,7 +580,9 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
                 // |b|^2) by less than 8 units of 2^-24 of |q|^2 + |limit|
                 const float d = unord32(lim);
                 const float t = (d - qn) + ((fabsf(d) + qn) * (1.0f / 524288.0f) + FLT_MIN);
-                thr = fabsf(t) <= FLT_MAX ? t : __int_as_float(0x7fffffff);
+                // 2 q.b may overflow where |b|^2 does not only for |q|^2 above FLT_MAX / 4:
+                // such a distance is -inf, which the sum without |q|^2 does not show
+                thr = fabsf(t) <= FLT_MAX && qn < FLT_MAX / 8 ? t : __int_as_float(0x7fffffff);
             }
         };
         set_limit(live ? *(volatile const uint32_t*)(a.bound + q) : 0u);
