@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
             mbar_init(&bar_empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&bar_accf[b], 1);
+            mbar_init(&bar_accf[b], 2);
             mbar_init(&bar_acce[b], 4);
         }
         mbar_init(&bar_drain, 1);
@@ -439,7 +439,13 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
                         parity ^= 1u;
                     }
                 }
-                if (ok) mma_commit(&bar_accf[b]);
+                if (ok) {
+                    mma_commit(&bar_accf[b]);
+                    // the epilogue reads the tile's bounds (thr_s) too, which arrived on bar_full:
+                    // this thread has waited there, and its own arrival hands that on (the
+                    // commit's arrival only says that the MMAs are done)
+                    mbar_arrive(&bar_accf[b]);
+                }
             }
             // every MMA issued has completed before the memory goes away
             mma_commit(&bar_drain);

@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&bar_empty[s])) : "memory");
         }
         for (int b = 0; b < 2; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&bar_accf[b])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" :: "r"(smem_addr(&bar_accf[b])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(&bar_acce[b])), "r"(EW) : "memory");
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&bar_a)) : "memory");
@@ -550,7 +550,14 @@ __global__ void __launch_bounds__(32 * (4 * MT + 2), 1) gt_kernel(const GtArgs a
                         parity ^= 1u;
                     }
                 }
-                if (ok) mma_commit(smem_addr(&bar_accf[b]));
+                if (ok) {
+                    mma_commit(smem_addr(&bar_accf[b]));
+                    // the epilogue reads the tile's norms too, which arrived on bar_full: this
+                    // thread has waited for them there, and its own arrival hands that on (the
+                    // commit's arrival only says that the MMAs are done)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
+                                 :: "r"(smem_addr(&bar_accf[b])) : "memory");
+                }
             }
             if (!ok) abort_flag = 1;
             consumed_s = consumed;
