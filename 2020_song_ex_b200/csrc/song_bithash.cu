@@ -648,9 +648,9 @@ song_status song_bithash_project(const float* R, int dim, int hash_bits, const f
     cudaStream_t st = nullptr;
     const size_t rb = (size_t)hash_bits * dim * 4, xb = (size_t)n * dim * 4,
                  cb = (size_t)n * words * 4;
-    cudaError_t e = cudaMalloc(&d_R, rb);
-    if (e == cudaSuccess) e = cudaMalloc(&d_x, xb);
-    if (e == cudaSuccess) e = cudaMalloc(&d_c, cb);
+    cudaError_t e = song::device_alloc((void**)&d_R, rb);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&d_x, xb);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&d_c, cb);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_R, R, rb, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_x, x, xb, cudaMemcpyHostToDevice, st);

@@ -226,9 +226,9 @@ song_status create_common(int kind, const void* rows, int64_t n, int dim, const 
     if (e == cudaSuccess) e = song::device_alloc(&x->d_base, (size_t)n * row_bytes);
     if (e == cudaSuccess)
         e = song::device_alloc((void**)&x->d_adj, (size_t)n * params->block_size * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&x->d_counter, 2 * kCounterRing * sizeof(unsigned));
+    if (e == cudaSuccess) e = song::device_alloc((void**)&x->d_counter, 2 * kCounterRing * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(x->d_counter, 0, 2 * kCounterRing * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMalloc(&x->d_err, 256);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&x->d_err, 256);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         cudaMemPoolProps pp = {};
@@ -282,7 +282,7 @@ cudaError_t grow(T** ptr, size_t* cap, size_t bytes) {
     cudaFree(*ptr);
     *ptr = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc((void**)ptr, bytes);
+    cudaError_t e = song::device_alloc((void**)ptr, bytes);
     if (e == cudaSuccess) *cap = bytes;
     return e;
 }
@@ -333,9 +333,9 @@ song_status attach_entry_hubs(song_index* x, const std::vector<int32_t>& hubs) {
     x->d_entry_norm = nullptr;
     x->entry_hpad = 0;
     x->entry_hubs.clear();
-    cudaError_t e = cudaMalloc(&x->d_entry_ids, (size_t)hpad * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&x->d_entry_tiles, (size_t)hpad * kp * 2);
-    if (e == cudaSuccess) e = cudaMalloc(&x->d_entry_norm, (size_t)hpad * 4);
+    cudaError_t e = song::device_alloc((void**)&x->d_entry_ids, (size_t)hpad * 4);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&x->d_entry_tiles, (size_t)hpad * kp * 2);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&x->d_entry_norm, (size_t)hpad * 4);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(x->d_entry_ids, ids.data(), (size_t)hpad * 4, cudaMemcpyHostToDevice,
                             x->stream);
@@ -823,7 +823,7 @@ song_status song_index_set_precision(song_index* x, int precision) {
     if (precision == SONG_PREC_FP8) {
         cudaFree(x->d_fp8_scale);
         x->d_fp8_scale = nullptr;
-        SONG_CUDA(cudaMalloc(&x->d_fp8_scale, (size_t)x->n * sizeof(float)), "scale alloc");
+        SONG_CUDA(song::device_alloc((void**)&x->d_fp8_scale, (size_t)x->n * sizeof(float)), "scale alloc");
     }
     SONG_CUDA(song::quantize_rows(precision, (const float*)x->d_base, x->n, x->dim, x->ld, *dst,
                                   row_bytes, x->d_fp8_scale, x->stream),
@@ -986,7 +986,7 @@ void song_learn_params_default(song_learn_params* p) {
 static song_status attach_model(song_index* x) {
     cudaFree(x->d_hubs);
     x->d_hubs = nullptr;
-    SONG_CUDA(cudaMalloc(&x->d_hubs, std::max<size_t>(1, x->hubs.size()) * 4), "hub alloc");
+    SONG_CUDA(song::device_alloc((void**)&x->d_hubs, std::max<size_t>(1, x->hubs.size()) * 4), "hub alloc");
     SONG_CUDA(cudaMemcpy(x->d_hubs, x->hubs.data(), x->hubs.size() * 4, cudaMemcpyHostToDevice), "hubs");
     SONG_CUDA(song::upload_half(x->entry_p, &x->d_entry_w), "entry weights");
     SONG_CUDA(song::upload_half(x->stop_p, &x->d_stop_w), "stop weights");
@@ -1009,7 +1009,7 @@ song_status song_index_learn(song_index* x, const song_learn_params* lp,
     if (cur != x->device) SONG_CUDA(cudaSetDevice(x->device), "cudaSetDevice");
     const int ef = clamp_ef(lp->ef, lp->k, x->p.pq_size);
     int32_t* d_ids = nullptr;
-    SONG_CUDA(cudaMalloc(&d_ids, (size_t)nq * lp->k * 4), "train ids alloc");
+    SONG_CUDA(song::device_alloc((void**)&d_ids, (size_t)nq * lp->k * 4), "train ids alloc");
     song::SearchArgs a;
     song_status s = make_args(x, d_train_queries, nq, lp->k, ef, d_ids, nullptr, &a);
     if (s != SONG_OK) {
@@ -1040,8 +1040,8 @@ song_status song_index_learn(song_index* x, const song_learn_params* lp,
         song_status s3 = attach_entry_hubs(x, perm);
         cudaError_t e3 = cudaSuccess;
         if (s3 == SONG_OK) {
-            e3 = cudaMalloc(&d_tc, (size_t)nq * song::kEntryK * 4);
-            if (e3 == cudaSuccess) e3 = cudaMalloc(&d_td, (size_t)nq * song::kEntryK * 4);
+            e3 = song::device_alloc((void**)&d_tc, (size_t)nq * song::kEntryK * 4);
+            if (e3 == cudaSuccess) e3 = song::device_alloc((void**)&d_td, (size_t)nq * song::kEntryK * 4);
             if (e3 != cudaSuccess) s3 = cuda_fail(e3, "entry candidates alloc");
         }
         if (s3 == SONG_OK) s3 = run_entry(x, d_train_queries, nq, d_tc, d_td, x->stream);

@@ -859,8 +859,8 @@ namespace song {
 // which keeps up to kPoolKeep bytes for the next call: a cudaMalloc and
 // cudaFree of the workspace took 0.6 - 1.3 ms per call, most of a small
 // call's time.  trim_workspaces gives the kept bytes back; destroying an
-// index does, and an allocation of an index or a graph build that fails does
-// before it tries again.
+// index does, and device_alloc does before it fails (a cudaMalloc of other
+// code has been seen to get them from the driver as well).
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[64] = {};
 constexpr uint64_t kPoolKeep = 1ull << 30;
@@ -1001,9 +1001,11 @@ cudaError_t exact_knn(const float* d_base, int64_t n, int64_t ldb, int dim, cons
         }
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, flags + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
+    // freed ahead of the synchronisation: a free that is still on its way keeps
+    // the memory from every other allocation until the stream is next waited for
+    const cudaError_t ef = cudaFreeAsync(ws, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     *err_out = h_err;
-    const cudaError_t ef = cudaFreeAsync(ws, st);
     return e != cudaSuccess ? e : ef;
 }
 
@@ -1043,10 +1045,10 @@ song_status song_exact_knn(const float* base, int64_t n, int dim, const float* q
     int32_t* d_i = nullptr;
     cudaStream_t st = nullptr;
     const size_t bb = (size_t)n * dim * 4, qb = (size_t)nq * dim * 4, ob = (size_t)nq * k;
-    cudaError_t e = cudaMalloc(&d_b, bb);
-    if (e == cudaSuccess) e = cudaMalloc(&d_q, qb);
-    if (e == cudaSuccess) e = cudaMalloc(&d_i, ob * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&d_d, ob * 4);
+    cudaError_t e = song::device_alloc((void**)&d_b, bb);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&d_q, qb);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&d_i, ob * 4);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&d_d, ob * 4);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_b, base, bb, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_q, queries, qb, cudaMemcpyHostToDevice, st);

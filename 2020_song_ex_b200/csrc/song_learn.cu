@@ -258,7 +258,7 @@ __global__ void entry_labels_staged(const float* __restrict__ base, int ld, int 
 
 template <typename T>
 cudaError_t dalloc(T** p, size_t count) {
-    return cudaMalloc((void**)p, std::max<size_t>(1, count) * sizeof(T));
+    return song::device_alloc((void**)p, std::max<size_t>(1, count) * sizeof(T));
 }
 
 // Adam training of one MLP on samples (X [M x kFeat], Y [M], W [M] nullable).
@@ -541,7 +541,7 @@ cudaError_t upload_half(const std::vector<float>& P, __half** d) {
     for (size_t i = 0; i < P.size(); ++i) h[i] = __float2half_rn(P[i]);
     cudaFree(*d);
     *d = nullptr;
-    cudaError_t e = cudaMalloc((void**)d, std::max<size_t>(1, h.size()) * sizeof(__half));
+    cudaError_t e = song::device_alloc((void**)d, std::max<size_t>(1, h.size()) * sizeof(__half));
     if (e == cudaSuccess) e = cudaMemcpy(*d, h.data(), h.size() * sizeof(__half), cudaMemcpyHostToDevice);
     return e;
 }

@@ -217,8 +217,8 @@ song_status song_server_create(song_index* index, const song_server_config* cfg,
     v->slots = (int)slots;
     cudaError_t e = cudaSetDevice(v->device);
     const size_t nk = (size_t)v->slots * cfg->max_k;
-    if (e == cudaSuccess) e = cudaMalloc(&v->d_ring, (size_t)v->slots * v->slot_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&v->d_ctrl, 64);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&v->d_ring, (size_t)v->slots * v->slot_bytes);
+    if (e == cudaSuccess) e = song::device_alloc((void**)&v->d_ctrl, 64);
     if (e == cudaSuccess) e = cudaMemset(v->d_ctrl, 0, 64);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // kst and cst do not wait for the legacy stream
     if (e == cudaSuccess) e = cudaHostAlloc(&v->h_stage, (size_t)v->slots * v->slot_bytes, cudaHostAllocDefault);
@@ -229,10 +229,10 @@ song_status song_server_create(song_index* index, const song_server_config* cfg,
     if (e == cudaSuccess) e = cudaHostAlloc(&v->h_trace, (size_t)v->slots * sizeof(song_query_trace), cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostAlloc(&v->h_done, (size_t)v->slots * 8, cudaHostAllocMapped);
     if (e == cudaSuccess && song::index_model_staged(index)) {
-        e = cudaMalloc(&v->d_scand, (size_t)v->slots * song::kEntryK * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&v->d_sdist, (size_t)v->slots * song::kEntryK * 4);
+        e = song::device_alloc((void**)&v->d_scand, (size_t)v->slots * song::kEntryK * 4);
+        if (e == cudaSuccess) e = song::device_alloc((void**)&v->d_sdist, (size_t)v->slots * song::kEntryK * 4);
         v->split_bytes = song::entry_split_scratch_bytes(128, v->num_sms);
-        if (e == cudaSuccess) e = cudaMalloc(&v->d_split, v->split_bytes);
+        if (e == cudaSuccess) e = song::device_alloc((void**)&v->d_split, v->split_bytes);
     }
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&v->kst, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&v->cst, cudaStreamNonBlocking);
