@@ -172,7 +172,12 @@ cudaError_t build_graph_device(int kind, const void* d_base, int64_t n, int dim,
     if (e == cudaSuccess && byte_rows(range, dim)) {
         u8_ld = u8_row_bytes(dim);
         e = workspace_alloc((void**)&u8, (size_t)n * u8_ld, st);
-        if (e == cudaSuccess)
+        if (e == cudaErrorMemoryAllocation) {  // only there for speed: the float rows give the same graph
+            cudaGetLastError();
+            u8 = nullptr;
+            e = cudaSuccess;
+        }
+        if (e == cudaSuccess && u8 != nullptr)
             e = convert_rows_u8(static_cast<const float*>(d_base), n, dim, ld, u8, u8_ld, st);
     }
     int64_t s = 1;
