@@ -944,6 +944,16 @@ cudaError_t exact_knn(const float* d_base, int64_t n, int64_t ldb, int dim, cons
     const size_t o_nth = take(um ? (size_t)nq * splits * 4 : 0);
     char* ws = nullptr;
     e = workspace_alloc(reinterpret_cast<void**>(&ws), total, st);
+    if (e == cudaErrorMemoryAllocation && nq > 2 * kM) {
+        // no room for the lists of all queries (512 or 2,048 bytes per query and
+        // split): half of them at a time, with the same results
+        cudaGetLastError();
+        const int half = (nq / 2 + 2 * kM - 1) / (2 * kM) * (2 * kM);
+        e = exact_knn(d_base, n, ldb, dim, d_q, half, ldq, k, d_ids, d_dists, st, err_out);
+        if (e != cudaSuccess || *err_out != 0) return e;
+        return exact_knn(d_base, n, ldb, dim, d_q + (int64_t)half * ldq, nq - half, ldq, k,
+                         d_ids + (int64_t)half * k, d_dists + (int64_t)half * k, st, err_out);
+    }
     if (e != cudaSuccess) return e;
     int* flags = reinterpret_cast<int*>(ws + o_flags);
     e = cudaMemsetAsync(flags, 0, 3 * sizeof(int), st);

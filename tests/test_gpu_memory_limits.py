@@ -2,8 +2,8 @@
 
 The workspace that the library keeps between calls is given back to
 allocations that would fail, and what is only there for speed (the byte copy
-of a build's rows) is not required: each call gives the result it gives with
-room to spare.
+of a build's rows, lists for all queries of an exact kNN at once) is not
+required: each call gives the result it gives with room to spare.
 """
 import numpy as np
 import pytest
@@ -120,3 +120,15 @@ def test_build_without_room_for_byte_rows(cuda, song):
         got = song.build_graph(rows, p)
     np.testing.assert_array_equal(got, want)
     give_back(song)
+
+
+def test_knn_without_room_for_all_lists(cuda, song):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(7)
+    b = torch.randn((1000, 8), device="cuda", generator=g)
+    q = torch.randn((200_000, 8), device="cuda", generator=g)  # lists of 410 MB
+    want, wd = knn_device(torch, song, b, q, 17)
+    give_back(song)
+    with NearlyFull(torch, 200):
+        ids, d = knn_device(torch, song, b, q, 17)
+    assert torch.equal(ids, want) and torch.equal(d, wd)
