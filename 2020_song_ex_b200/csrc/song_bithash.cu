@@ -19,7 +19,9 @@
 // bound has the sign of m; the others (about one in 1,300 at 256 dimensions
 // of Gaussian data) are summed as above.  Every comparison with a NaN, an
 // overflow or a norm near the underflow range counts as "near zero", and if a
-// bounded wait gives up the CTA sums all of its remaining bits that way.
+// bounded wait gives up the CTA sums all of its remaining bits that way.  The
+// norms are each vector's and each hyperplane's own: one that has no bound
+// sends its own bits to the sums and no others.
 //
 // One CTA takes 128 hyperplanes (4 code words), their BF16 parts resident in
 // shared memory up to 288 dimensions, and walks over tiles of 128 vectors;
@@ -33,13 +35,19 @@
 //     code words with two funnel shifts per bit, free the buffer and then sum
 //     the near-zero bits of their tile, one per lane, under the next tile's
 //     products.
+// A tile where a warp finds more than kDense such bits is marked and summed
+// whole by all warps at the end (sum_left), as all tiles are above kTensorDim
+// dimensions.  So the time does not hang on the data: 100,000 x 256 -> 512 bits
+// 0.17 ms, with a zero hyperplane 0.17, a tiny one 0.28, one tiny vector in 32
+// 0.64, all vectors tiny 1.29 (the sums of all bits by a kernel made for them
+// 1.35; with the largest norm for all 128 hyperplanes and each lane summing its
+// own vector's bits 14.0, 14.0, 5.3 and 14.0 ms).
 // The floor is 3 products per multiply of the projection on the tensor cores
 // (0.14 ms for 290,000 x 256 -> 512 bits) or one pass over x (0.05 ms).  The
 // sums of all bits on the CUDA cores, 255 registers per thread and 8 warps per
-// SM, took 3.81 ms; this takes 0.47 ms (50,000 x 960 -> 1,024 bits 4.93 -> 1.13
-// ms, 1,000 x 256 -> 512 bits 41 -> 23 us).  What bounds it now is the
-// converters' loads of x: without products 0.41 ms, without near-zero sums
-// 0.43 ms.
+// SM, took 3.81 ms; this takes 0.41 ms.  What bounds it is the converters' loads
+// of x (in a form that took 0.47 ms: without products 0.41, without near-zero
+// sums 0.43).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
@@ -73,6 +81,18 @@ constexpr int kThrSlots = 8;          // the converters run at most 8 tiles ahea
 constexpr int kEpi = 8, kConv = 8;    // epilogue and converter warps
 constexpr int kThreads = 32 * (kEpi + 1 + kConv);
 constexpr int kItems = 128;           // near-zero bits a warp collects before it sums them
+// With more near-zero bits among a warp's 4,096 the whole tile is summed at the
+// end: 32 of them take about 16,000 cycles here (dependent loads and sums), the
+// tile 80,000 there, by all warps.
+constexpr int kDense = 256;
+// The bound grows with the dimension and the sums' spread against it shrinks: 4 %
+// of the bits are near zero at 4,096 dimensions (10,000 vectors -> 256 bits 1.59
+// ms, 1.92 by a kernel of sequential sums) and 7 % at 6,000, where most tiles
+// would be summed whole after the products (4.9 ms; 2.6 without them).
+constexpr int kTensorDim = 4096;
+constexpr int kSeqBits = 1024;        // marks of such tiles (each for a run of tiles when there are more)
+constexpr float kMinNorm2 = 1e-24f;   // smaller squared norms have no bound: products of two such vectors
+                                      // stay far above what underflow can take away (2^-126 a product)
 constexpr long long kWaitCycles = 4000000000LL;  // about 2 s
 
 // Bound on |m - s| / (|x| |r|), with S = sum |x_i r_i| <= |x| |r|, u = 2^-24:
@@ -249,10 +269,96 @@ struct BhArgs {
     int words;        // code words per vector
     int groups;       // CTAs side by side: ceil(words / kWords)
     int per_group;    // CTAs of one group of words
-    int64_t tiles;    // tiles of 128 vectors
+    int tv;           // vectors per tile: kTV, or (without tensor) a half or a quarter of it
+    int64_t tiles;    // tiles of tv vectors
     int nch;
     float factor;     // error_factor(dim)
+    bool tensor;      // signs from the tensor cores (dim <= kTensorDim)
 };
+
+// What sum_left needs, in shared memory: nothing of it is kept in registers
+// through the kernel's main loops.
+struct Left {
+    BhArgs a;
+    int64_t tiles, first;             // this CTA's tiles: first + i * a.per_group
+    int group, shift;                 // mark of tile i: i >> shift
+    uint32_t marks[kSeqBits / 32];
+};
+
+// All bits of the marked tiles by the reference's sums, the whole CTA: 16 warps
+// of 32 vectors x 32 hyperplanes, a lane 4 x 8 of them (12 values from shared
+// memory for 32 products; with 32 hyperplanes per lane the loads took twice the
+// time of the sums).  Chunks of 32 dimensions go through shared memory
+// transposed, the next one in flight in registers.
+__device__ __noinline__ void sum_left(const Left& l, float* sh) {
+    constexpr int kPer = kTV * kDC / 512;  // elements per thread and side
+    constexpr int kPad = 128 + 4;
+    float *xs = sh, *rs = sh + kDC * kPad;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int vb = (warp >> 2) * 32 + 4 * (lane >> 2), hb = (warp & 3) * 32 + 8 * (lane & 3);
+    const int dim = l.a.R.dim, nr = (int)min((int64_t)kTB, l.a.R.count - (int64_t)l.group * kTB);
+    const bool mine = t < 512 && (warp & 3) * 32 < nr && (warp >> 2) * 32 < l.a.tv;
+    const float* R = l.a.R.p + (int64_t)(l.group * kTB + warp) * l.a.R.ld + lane;
+    for (int64_t i = 0; i < l.tiles; ++i) {
+        const int m = (int)(i >> l.shift);
+        if (!((l.marks[m >> 5] >> (m & 31)) & 1u)) continue;
+        const int64_t v0 = (l.first + i * l.a.per_group) * l.a.tv;
+        const float* x = l.a.x.p + (v0 + warp) * l.a.x.ld + lane;
+        const int nx = (int)min((int64_t)l.a.tv, l.a.x.count - v0);
+        float px[kPer], pr[kPer];
+        auto fetch = [&](int d0) {
+            const bool in = t < 512 && d0 + lane < dim;
+#pragma unroll
+            for (int e = 0; e < kPer; ++e) {
+                px[e] = in && e * 16 + warp < nx ? __ldg(x + e * 16 * l.a.x.ld + d0) : 0.0f;
+                pr[e] = in && e * 16 + warp < nr ? __ldg(R + e * 16 * l.a.R.ld + d0) : 0.0f;
+            }
+        };
+        float s[4][8];
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[p][j] = 0.0f;
+        fetch(0);
+        for (int d0 = 0; d0 < dim; d0 += kDC) {
+            __syncthreads();  // the chunk before has been read
+            if (t < 512) {
+#pragma unroll
+                for (int e = 0; e < kPer; ++e) {
+                    xs[lane * kPad + e * 16 + warp] = px[e];
+                    rs[lane * kPad + e * 16 + warp] = pr[e];
+                }
+            }
+            __syncthreads();
+            if (d0 + kDC < dim) fetch(d0 + kDC);
+            if (!mine) continue;
+            const int cl = min(kDC, dim - d0);
+#pragma unroll 2
+            for (int d = 0; d < cl; ++d) {
+                const float4 x4 = *reinterpret_cast<const float4*>(xs + d * kPad + vb);
+                const float4 ra = *reinterpret_cast<const float4*>(rs + d * kPad + hb);
+                const float4 rb = *reinterpret_cast<const float4*>(rs + d * kPad + hb + 4);
+                const float xv[4] = {x4.x, x4.y, x4.z, x4.w};
+                const float rv[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) s[p][j] = __fadd_rn(s[p][j], __fmul_rn(rv[j], xv[p]));
+            }
+        }
+        uint32_t* codes = l.a.codes + v0 * l.a.ldc + l.group * kWords + (warp & 3);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            uint32_t bits = 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bits |= (s[p][j] > 0.0f ? 1u : 0u) << j;
+            bits <<= 8 * (lane & 3);
+            bits |= __shfl_xor_sync(FULL, bits, 1);
+            bits |= __shfl_xor_sync(FULL, bits, 2);
+            if (mine && (lane & 3) == p && vb + p < nx) codes[(vb + p) * l.a.ldc] = bits;
+        }
+    }
+}
 
 template <bool RES>
 __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
@@ -260,11 +366,12 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
     constexpr uint32_t kStageBytes = (RES ? 2 : 4) * kBlock;  // xh, xl (, rh, rl)
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar_full[kStages], bar_empty[kStages], bar_accf[2], bar_acce[2], bar_drain;
-    __shared__ float thr_s[kThrSlots][kTV];
+    __shared__ float thr_s[kThrSlots][kTV];  // |x| of the vectors of the tiles in flight
     __shared__ uint16_t item_s[kEpi][kItems];
     __shared__ uint32_t fix_s[kEpi][32 * kWords];
+    __shared__ Left left_s;
     __shared__ uint32_t tslot;
-    __shared__ unsigned rn2_s;  // largest squared norm of the CTA's hyperplanes (ordered bits)
+    __shared__ __align__(16) float rn_s[kTB];  // error_factor * |r| of each hyperplane
     __shared__ volatile int abort_flag, never;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     unsigned char* r_blocks = smem;                                       // RES: [hi, lo][nch][kBlock]
@@ -273,12 +380,22 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
 
     const int group = blockIdx.x % a.groups;
     const int64_t first = blockIdx.x / a.groups;
-    const int64_t mytiles = first < a.tiles ? (a.tiles - first + a.per_group - 1) / a.per_group : 0;
+    int64_t mytiles = first < a.tiles ? (a.tiles - first + a.per_group - 1) / a.per_group : 0;
+    if (tid < kSeqBits / 32) left_s.marks[tid] = a.tensor ? 0u : FULL;
+    if (tid == 0) {
+        left_s.a = a;
+        left_s.tiles = mytiles;
+        left_s.first = first;
+        left_s.group = group;
+        left_s.shift = 0;
+        while ((mytiles >> left_s.shift) >= kSeqBits) ++left_s.shift;
+    }
+    if (!a.tensor) mytiles = 0;  // all tiles are left over
     Rows R = a.R;
     R.p += (int64_t)group * kTB * R.ld;
     R.count = min((int64_t)kTB, R.count - (int64_t)group * kTB);
 
-    if (warp == 0) {
+    if (a.tensor && warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_addr(&tslot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -294,34 +411,35 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
         }
         mbar_init(&bar_drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        rn2_s = 0u;
         abort_flag = 0;
         never = 0;
     }
     __syncthreads();
-    // the hyperplanes' norms and (RES) operand blocks: a warp per 8 of them
+    // the hyperplanes' norms and (RES) operand blocks: a warp per 8 of them.  A
+    // hyperplane without a bound (norm not finite or near underflow) has all its
+    // bits summed (+inf); one of zeros has all clear whatever the vector (-inf:
+    // the bound is below every |m|, and m is 0)
     const int kd = lane_dim(lane);
-    {
-        float rn2 = 0.0f;
-        bool bad = false;
-        for (int r8 = warp; r8 < kTB / 8; r8 += kThreads / 32) {
-            const int r = r8 * 8 + lane_row(lane);
-            float q = 0.0f;
-            for (int c = 0; c < a.nch; ++c) {
-                float v[8];
-                load8(R, r, c * kDC + kd, v);
+    for (int r8 = a.tensor ? warp : kTB; r8 < kTB / 8; r8 += kThreads / 32) {
+        const int r = r8 * 8 + lane_row(lane);
+        float q = 0.0f;
+        unsigned any = 0u;
+        for (int c = 0; c < a.nch; ++c) {
+            float v[8];
+            load8(R, r, c * kDC + kd, v);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) q = fmaf(v[e], v[e], q);
-                if constexpr (RES) store_split(r_blocks + (size_t)c * kBlock, r_lo, r8, lane, v);
+            for (int e = 0; e < 8; ++e) {
+                q = fmaf(v[e], v[e], q);
+                any |= __float_as_uint(v[e]) << 1;
             }
-            q += __shfl_xor_sync(FULL, q, 1);
-            q += __shfl_xor_sync(FULL, q, 16);
-            // near underflow the bound does not hold: none then (infinite)
-            if (r < R.count && !(q >= 1e-30f)) bad = true;
-            rn2 = fmaxf(rn2, q);
+            if constexpr (RES) store_split(r_blocks + (size_t)c * kBlock, r_lo, r8, lane, v);
         }
-        if (bad) rn2 = INFINITY;
-        atomicMax(&rn2_s, __float_as_uint(rn2));
+#pragma unroll
+        for (int o = 1; o <= 16; o <<= 4) {
+            q += __shfl_xor_sync(FULL, q, o);
+            any |= __shfl_xor_sync(FULL, any, o);
+        }
+        if ((lane & 17) == 0) rn_s[r] = any == 0u ? -INFINITY : (q >= kMinNorm2 ? a.factor * sqrtf(q) : INFINITY);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -332,7 +450,6 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
     if (warp > kEpi) {
         // ---- converters ----
         const int w = warp - kEpi - 1;
-        const float rbound = a.factor * sqrtf(__uint_as_float(rn2_s));
         constexpr int kT = RES ? 2 : 4;  // 8 vectors each, then (streamed) 8 hyperplanes each
         const int r0 = w * 8 + lane_row(lane);
         const int64_t total = mytiles * a.nch;
@@ -381,10 +498,10 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
                     any1 |= __shfl_xor_sync(FULL, any1, o);
                 }
                 // a zero vector's sums are zero (every bit certain: 0 > -1, clear); a norm
-                // near underflow has no bound
+                // near underflow, as one that is not finite, has no bound
                 if ((lane & 17) == 0) {
-                    thr_s[slot][r0] = any0 == 0u ? -1.0f : (q0 >= 1e-30f ? rbound * sqrtf(q0) : INFINITY);
-                    thr_s[slot][r0 + 64] = any1 == 0u ? -1.0f : (q1 >= 1e-30f ? rbound * sqrtf(q1) : INFINITY);
+                    thr_s[slot][r0] = any0 == 0u ? -1.0f : (q0 >= kMinNorm2 ? sqrtf(q0) : INFINITY);
+                    thr_s[slot][r0 + 64] = any1 == 0u ? -1.0f : (q1 >= kMinNorm2 ? sqrtf(q1) : INFINITY);
                 }
                 slot = (slot + 1) % kThrSlots;
                 q0 = q1 = 0.0f;
@@ -448,8 +565,10 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
                 }
             }
             // every MMA issued has completed before the memory goes away
-            mma_commit(&bar_drain);
-            mbar_wait(smem_addr(&bar_drain), 0u, &never);
+            if (a.tensor) {
+                mma_commit(&bar_drain);
+                mbar_wait(smem_addr(&bar_drain), 0u, &never);
+            }
         }
     } else {
         // ---- epilogue: set b reads accumulator buffer b; thread = vector = TMEM lane ----
@@ -476,10 +595,16 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
                         tmem_ld16(acc + (uint32_t)(kTB + w * 32 + h * 16), x);
                         tmem_wait16(m, x);
 #pragma unroll
-                        for (int j = 15; j >= 0; --j) {  // bit j of the half: sign of 0 - sum, sign of bound - |sum|
-                            const float sum = __fadd_rn(__uint_as_float(m[j]), __uint_as_float(x[j]));
-                            bits = __funnelshift_l(__float_as_uint(__fsub_rn(0.0f, sum)), bits, 1);
-                            sure = __funnelshift_l(__float_as_uint(__fsub_rn(thr, fabsf(sum))), sure, 1);
+                        for (int j4 = 3; j4 >= 0; --j4) {
+                            const float4 rn4 = *reinterpret_cast<const float4*>(rn_s + w * 32 + h * 16 + 4 * j4);
+                            const float rn[4] = {rn4.x, rn4.y, rn4.z, rn4.w};
+#pragma unroll
+                            for (int e = 3; e >= 0; --e) {  // sign of 0 - sum, sign of bound - |sum|
+                                const int j = 4 * j4 + e;
+                                const float sum = __fadd_rn(__uint_as_float(m[j]), __uint_as_float(x[j]));
+                                bits = __funnelshift_l(__float_as_uint(__fsub_rn(0.0f, sum)), bits, 1);
+                                sure = __funnelshift_l(__float_as_uint(fmaf(thr, rn[e], -fabsf(sum))), sure, 1);
+                            }
                         }
                     }
                     word[w] = bits;
@@ -511,30 +636,27 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
             }
             const int total = __shfl_sync(FULL, before, 31);
             before -= cnt;
-            if (total > kItems) {  // many (data made of near-zero sums): each lane sums its own
+            if (total > kDense) {  // many (vectors without a bound, or so many dimensions that it is wide)
+                const int m = (int)(i >> left_s.shift);
+                if (lane == 0) atomicOr(&left_s.marks[m >> 5], 1u << (m & 31));
+                continue;
+            } else if (total > 0) {  // few: spread over the lanes, kItems at a time
 #pragma unroll
-                for (int w = 0; w < kWords; ++w)
-                    while (unc[w]) {
-                        const int j = __ffs(unc[w]) - 1;
-                        unc[w] &= unc[w] - 1u;
-                        const float s = dot_seq(R.p + (int64_t)(w * 32 + j) * R.ld, a.x.p + v * a.x.ld, R.dim, vec);
-                        word[w] = (word[w] & ~(1u << j)) | ((s > 0.0f ? 1u : 0u) << j);
+                for (int w = 0; w < kWords; ++w) fix_s[warp][lane * kWords + w] = word[w] & ~unc[w];
+                for (int done = 0; done < total; done += kItems) {
+#pragma unroll
+                    for (int w = 0; w < kWords; ++w)
+                        for (; unc[w] && before < done + kItems; unc[w] &= unc[w] - 1u)
+                            item_s[warp][before++ - done] = (uint16_t)(lane * kTB + w * 32 + __ffs(unc[w]) - 1);
+                    __syncwarp();
+                    for (int t = lane; t < min(kItems, total - done); t += 32) {
+                        const int it = item_s[warp][t], l = it / kTB, j = it % kTB;
+                        const float s = dot_seq(R.p + (int64_t)j * R.ld,
+                                                a.x.p + (v0 + (warp & 3) * 32 + l) * a.x.ld, R.dim, vec);
+                        if (s > 0.0f) atomicOr(&fix_s[warp][l * kWords + (j >> 5)], 1u << (j & 31));
                     }
-            } else if (total > 0) {  // few: spread over the lanes
-#pragma unroll
-                for (int w = 0; w < kWords; ++w) {
-                    fix_s[warp][lane * kWords + w] = word[w] & ~unc[w];
-                    for (unsigned m = unc[w]; m; m &= m - 1u)
-                        item_s[warp][before++] = (uint16_t)(lane * kTB + w * 32 + __ffs(m) - 1);
+                    __syncwarp();
                 }
-                __syncwarp();
-                for (int t = lane; t < total; t += 32) {
-                    const int it = item_s[warp][t], l = it / kTB, j = it % kTB;
-                    const float s = dot_seq(R.p + (int64_t)j * R.ld,
-                                            a.x.p + (v0 + (warp & 3) * 32 + l) * a.x.ld, R.dim, vec);
-                    if (s > 0.0f) atomicOr(&fix_s[warp][l * kWords + (j >> 5)], 1u << (j & 31));
-                }
-                __syncwarp();
 #pragma unroll
                 for (int w = 0; w < kWords; ++w) word[w] = fix_s[warp][lane * kWords + w];
                 __syncwarp();
@@ -550,8 +672,9 @@ __global__ void __launch_bounds__(kThreads, 1) bithash_kernel(const BhArgs a) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 0)
+    if (a.tensor && warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512) : "memory");
+    sum_left(left_s, reinterpret_cast<float*>(smem));  // the ring's memory is free now
 }
 
 song_status fail(song_status s, const char* msg) { return song::set_error(s, msg); }
@@ -588,7 +711,19 @@ cudaError_t launch_bithash(const float* d_R, int dim, int hash_bits, const float
     a.ldc = ldc;
     a.words = hash_bits / 32;
     a.groups = (a.words + kWords - 1) / kWords;
-    a.tiles = (n + kTV - 1) / kTV;
+    a.tensor = dim <= kTensorDim;
+    a.tv = kTV;
+    if (!a.tensor) {
+        // the height with the least time: tiles of the busiest CTA, each as long as
+        // its height and about 96 more (the chunks' loads and barriers: 1,000 x
+        // 100,000 -> 256 bits 21.4 ms at 128, 12.1 at 32; 10,000 x 6,000 2.5 ms at
+        // 128, two tiles, 3.2 at 64, three)
+        const int64_t ctas = std::max(1, num_sms / a.groups);
+        auto cost = [&](int tv) { return ((n + tv - 1) / tv + ctas - 1) / ctas * (tv + 96); };
+        for (int tv = kTV / 2; tv >= 32; tv /= 2)
+            if (cost(tv) < cost(a.tv)) a.tv = tv;
+    }
+    a.tiles = (n + a.tv - 1) / a.tv;
     a.per_group = (int)std::min<int64_t>(std::max(1, num_sms / a.groups), a.tiles);
     a.nch = (dim + kDC - 1) / kDC;
     a.factor = error_factor(dim);
