@@ -101,7 +101,10 @@ constexpr long long kWaitCycles = 4000000000LL;  // about 2 s
 //  * each tcgen05.mma adds 16 exact products and the accumulator, every one
 //    of them off by at most 2^-23 of the largest when they are aligned: 17 *
 //    2^-23 S per instruction, dim / 16 of them for xh.rh; the other
-//    accumulator holds terms 2^-8 as large (twice as many instructions);
+//    accumulator holds terms 2^-8 as large (twice as many instructions).  How
+//    far it rounds is an assumption, no document says: sums made to lose most
+//    (a large part taken back) and 5 million Gaussian ones still had every sign
+//    right with an eighth of this bound, and not with a 64th;
 //  * the reference's sum itself: dim products and sums, below (dim + 1) u S,
 //    and the final m = main + cross below 2 u S.
 // The norms are FP32 sums of squares: 2^-10 covers their rounding.
