@@ -303,14 +303,11 @@ static cudaError_t launch_instance(KernelSel ks, int kind, const SearchArgs& arg
             fn = ks.fn_tmd;
             tm_per_sm = p2;
         }
+        // four such warps leave no room for the query: the instances that read it
+        // from global memory
         if (tm_per_sm < 1 && ks.query_smem && kind == SONG_KIND_L2 && a.prec == SONG_PREC_FP32 &&
-            args.dim <= kU8MaxDim) {
-            // four such warps leave no room for the query: read it from global memory
-            SearchArgs by_row = args;
-            by_row.u8 = reinterpret_cast<const uint8_t*>(1);  // picks the byte-row instance ...
-            const KernelSel no_query = pick_l2(by_row, false);
-            return launch_instance(no_query, kind, args, num_sms, stream);  // ... which finds no byte rows
-        }
+            args.dim <= kU8MaxDim)
+            return launch_instance(pick_l2(args, false, true), kind, args, num_sms, stream);
         if (tm_per_sm < 1) return cudaErrorInvalidConfiguration;
     } else {
         // Up to 8 warps per CTA while the CTA's shared memory stays within a

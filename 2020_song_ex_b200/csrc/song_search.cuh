@@ -2228,11 +2228,22 @@ KernelSel reg_queues(const SearchArgs& a) {
     return KernelSel();
 }
 
+// The plain instance for a.cap slots.
+template <int KIND, int NE, int DT>
+KernelSel by_cap(const SearchArgs& a, bool reg) {
+    if (reg) return reg_queues<KIND, NE, DT, 0>(a);
+    if (a.cap <= 1024) return ksel<KIND, NE, 1, DT>();
+    if (a.cap <= 2048) return ksel<KIND, NE, 2, DT>();
+    if (a.cap <= 4096) return ksel<KIND, NE, 4, DT>();
+    return KernelSel();
+}
+
 }  // namespace
 
 // Instances by file (song_search_*.cu).  reg: queues in registers; an empty
 // selection means none for these arguments.
-KernelSel pick_l2(const SearchArgs& a, bool reg);
+// query_global: an instance that can read the query from global memory.
+KernelSel pick_l2(const SearchArgs& a, bool reg, bool query_global = false);
 KernelSel pick_lowp(const SearchArgs& a, bool reg);
 KernelSel pick_hamming(const SearchArgs& a, bool reg);
 KernelSel pick_learned(const SearchArgs& a, bool reg);

@@ -3,17 +3,6 @@
 
 namespace song {
 
-namespace {
-template <int KIND, int NE, int DT>
-KernelSel by_cap(const SearchArgs& a, bool reg) {
-    if (reg) return reg_queues<KIND, NE, DT, 0>(a);
-    if (a.cap <= 1024) return ksel<KIND, NE, 1, DT>();
-    if (a.cap <= 2048) return ksel<KIND, NE, 2, DT>();
-    if (a.cap <= 4096) return ksel<KIND, NE, 4, DT>();
-    return KernelSel();
-}
-}  // namespace
-
 KernelSel pick_hamming(const SearchArgs& a, bool reg) {
     switch (a.ld) {
         case 4: return by_cap<1, 1, 0>(a, reg);
