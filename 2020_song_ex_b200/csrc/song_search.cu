@@ -356,10 +356,15 @@ cudaError_t launch_search(int kind, const SearchArgs& args, int num_sms, cudaStr
     // Queues in registers, unless they are too long or four warps' filters and
     // ids do not fit in shared memory.  Up to 160 slots they are faster at any
     // number of queries (10,000 of 128 integers: ef 64 1.29 -> 1.09 ms, ef 128
-    // 2.07 -> 1.95, ef 150 2.30 -> 2.25; one at ef 150 611 -> 511 us).  Up to 256
-    // the work per operation passes that of the group summaries and only the
-    // shorter chain remains, which wins while the SMs are nearly empty: 592
-    // queries at ef 256 1,460 -> 1,392 us, but 2,368 1,753 -> 1,876.
+    // 2.07 -> 1.95, ef 150 2.30 -> 2.25; one at ef 150 611 -> 511 us; 60, 120 and
+    // 150 slots and 1 to 10,000 queries of the other row types, too: float 1-33 %,
+    // BF16 and FP8 up to 10 %, Hamming 7-23 %, learned 5-36 %).  Up to 256 the work per
+    // operation passes that of the group summaries and only the shorter chain
+    // remains, which wins while the SMs are nearly empty.  200 and 256 slots, 1 to
+    // 592 queries / 10,000, time of the others over theirs: 128 integers 1.04-1.07
+    // / 0.87, float rows 1.12-1.22 / 0.99-1.01, BF16 1.02 / 0.98, FP8 1.00 / 0.97,
+    // Hamming 1.08-1.12 / 0.90-0.92, learned integers 1.05-1.08 / 0.94, learned
+    // float rows 0.98-1.00 / 1.01, learned BF16 1.04-1.05 / 1.08.
     const KernelSel reg = pick_kernel(kind, args, true);
     if (reg.fn != nullptr) {
         SearchArgs a = args;
