@@ -35,6 +35,10 @@
 //     code words with two funnel shifts per bit, free the buffer and then sum
 //     the near-zero bits of their tile, one per lane, under the next tile's
 //     products.
+// Two buffers of two accumulators are all 512 TMEM columns: beside a search on
+// another stream, whose CTAs keep their queues in TMEM, a CTA starts when those
+// on its SM have ended (it needs the SM's shared memory and registers too), and
+// the search's next ones wait for it.  Neither allocates twice: the waits end.
 // A tile where a warp finds more than kDense such bits is marked and summed
 // whole by all warps at the end (sum_left), as all tiles are above kTensorDim
 // dimensions.  So the time does not hang on the data: 100,000 x 256 -> 512 bits

@@ -56,6 +56,12 @@
 // (distance, id), ties broken by the lower id -- depends neither on the
 // split nor on the order in which thresholds are seen.
 //
+// A CTA takes an SM for itself: with two query tiles all 512 TMEM columns, and
+// nearly all shared memory.  Beside a search on another stream, whose CTAs keep
+// their queues in TMEM, it starts when those on its SM have ended; the search's
+// next CTAs wait likewise.  Each kernel allocates once, holding nothing else that
+// the others wait for, so these waits end.
+//
 // Every wait is bounded (about two seconds): a role that gives up raises the
 // CTA's abort flag and the error word, the others leave their loops, copies
 // still in flight and MMAs still running are waited for (again bounded), and
