@@ -27,7 +27,7 @@ comes from the library's GPU builder.  ``config.graph`` says which.
 
 Output: ONE compact JSON line on stdout (rank 0; a few KB at most).  Curves,
 sweeps, per-step times and the serving points go to a side file
-(``--details``, default ``gpurun_out/bench_details.json``) and to stderr.
+(``--details``, default ``bench_details.json`` beside this file) and to stderr.
 ``value`` is device-resident QPS of the fastest form meeting the recall
 target (queries and graph already in HBM); ``e2e`` is the same through the
 host C-ABI call (pinned host queries, H2D + kernels + D2H timed).
@@ -1340,7 +1340,7 @@ def main(argv=None):
     ap.add_argument("--steps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", choices=("ours", "reference"), default="ours")
-    ap.add_argument("--details", default=os.path.join(ROOT, "gpurun_out", "bench_details.json"),
+    ap.add_argument("--details", default=os.path.join(ROOT, "bench_details.json"),
                     help="side file for curves, sweeps and per-step times ('' = none)")
     ap.add_argument("--graph", choices=("auto", "gpu", "ref"), default="auto",
                     help="auto: the reference arm's graph when present, else the GPU builder")
