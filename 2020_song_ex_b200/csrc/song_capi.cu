@@ -580,8 +580,8 @@ song_status host_search(song_index* x, int kind, const void* queries, int nq, in
     // Per batch: copy in, search, copy out, on the index's stream with one
     // synchronisation at the end of the batch; the copy and kernel times come
     // from events between them, for callers that ask for times: four records and
-    // three reads of a batch were a sixth of a one-query call (251 -> 183 us
-    // with them, 163 us without; 100,000 x 128, queue 50).
+    // three reads take about 20 us of a one-query call (100,000 x 128: 208 -> 190
+    // us without them at queue 50, 388 -> 366 at queue 150).
     const bool timed = timing != nullptr;
     for (int off = 0; off < nq; off += chunk) {
         const int bs = std::min(chunk, nq - off);

@@ -46,8 +46,8 @@
 // of dependent shared accesses, one query tile of 4 warps per SM and a
 // separate threshold per split.  Whole calls: 10,000 queries x 1M x 128
 // integers at k = 10 17.6 -> 3.7 ms (the kernel 17.3 -> 3.5 ms, 0.73 PFLOP/s),
-// at k = 100 36.7 -> 7.3 ms; 777 x 99,991 x 100 floats at k = 100 2.2 -> 0.44
-// ms; 50 x 5,000 x 24 at k = 1 0.71 -> 0.10 ms.
+// at k = 100 36.7 -> 7.3 ms; 777 x 99,991 x 100 floats at k = 100 2.2 - 3.3 ms
+// (varying with its allocations) -> 0.44; 50 x 5,000 x 24 at k = 1 0.71 -> 0.10.
 //
 // A key that ties a split's own threshold has a larger id than the k kept
 // (bases are visited in increasing id order) and is dropped; one that ties

@@ -292,9 +292,10 @@ song_status song_bithash_project_device(const float* d_R, int dim, int hash_bits
  * (distance, id), -1 / +inf when n < k.  1 <= k <= 128.
  * The device form takes device buffers (row strides ldb, ldq in floats) and
  * returns when the result is on the device (it synchronises `stream`).  Up to
- * 1 GiB of its device workspace per GPU is kept for the next call; destroying
- * an index gives it back, and so does an allocation of this library that
- * would fail otherwise.
+ * 1 GiB of its device workspace per GPU is kept, unused, for the next call;
+ * destroying an index gives it back, and so does an allocation of this library
+ * that would fail otherwise.  Where the lists of all queries do not fit the
+ * device, the queries are taken in parts with the same results.
  */
 song_status song_exact_knn_device(const float* d_base, int64_t n, int64_t ldb, int dim,
                                   const float* d_queries, int nq, int64_t ldq, int k,
