@@ -92,3 +92,25 @@ def test_time_does_not_hang_on_them(cuda, song):
     x[::32] *= 1e-20
     assert ms(x, R0) < 6 * base
     assert ms(x0 * 1e-20, R0) < 25 * base
+
+
+def test_more_tiles_than_marks(cuda, song):
+    """More than 1,024 tiles per CTA: a mark stands for a run of tiles.  The
+    codes of all vectors at once are those of slices that need no runs."""
+    torch = cuda
+    n, dim, bits = 1_300_000, 8, 2048
+    h = song.BitHash(dim, 4, bits)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.randn((n, dim), device="cuda", generator=g)
+    for tile in torch.randint(0, n // 128, (300,), generator=torch.Generator().manual_seed(3)).tolist():
+        x[tile * 128:tile * 128 + 100] *= 1e-20
+    x[-40:] *= 1e-20
+    R = torch.from_numpy(h.R).cuda()
+    R[7] = 0.0
+    whole = torch.full((n, bits // 32), -1, dtype=torch.int32, device="cuda")
+    part = torch.full((n, bits // 32), -2, dtype=torch.int32, device="cuda")
+    h.project_device(R, x, n, whole, stream=torch.cuda.current_stream())
+    for s in range(0, n, 100_000):
+        m = min(100_000, n - s)
+        h.project_device(R, x[s:s + m], m, part[s:s + m], stream=torch.cuda.current_stream())
+    assert torch.equal(whole, part)
